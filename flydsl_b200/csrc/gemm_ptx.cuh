@@ -84,6 +84,11 @@ __device__ __forceinline__ bool elect_one() {
   asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
   return p != 0;
 }
+// All lanes of a warp wait together.
+__device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status, int code,
+                                          unsigned backoff_ns = 0) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code, backoff_ns));
+}
 __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, int c1) {
   asm volatile(
       "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -94,6 +99,39 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
+}
+// Routing of the launch.  A null sorted_ids is the identity routing of the dense GEMM: sorted row r is row r, every
+// row block belongs to expert 0, and all row blocks are in use -- no tables to write first.
+__device__ __forceinline__ int routed_rows(const GemmArgs& a) {
+  const int cap = a.size_expert_ids * a.tile_m;
+  return a.sorted_ids != nullptr ? min(__ldg(a.num_valid_ids), cap) : cap;
+}
+__device__ __forceinline__ int block_expert(const GemmArgs& a, int b) {
+  return a.sorted_ids != nullptr ? __ldg(a.sorted_expert_ids + b) : 0;
+}
+__device__ __forceinline__ int sorted_id(const GemmArgs& a, int r) {
+  return a.sorted_ids != nullptr ? __ldg(a.sorted_ids + r) : min(r, a.num_tokens);   // num_tokens: a pad row
+}
+// Four rows by index (a box of one row, 128 bytes of K each) to four consecutive 128-byte rows of the tile; the
+// 128-byte swizzle goes by the shared-memory address, so dst only has to be a multiple of 512 bytes.
+__device__ __forceinline__ void tma_gather4(uint32_t dst, const CUtensorMap* map, uint32_t bar, int c0, const int* r) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
+      ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
+}
+// Row of the activations that sorted row `first + i` stands for, i = 0..3 (row 0 for pad rows and rows beyond
+// `end`: their results are never used).
+__device__ __forceinline__ void gather_rows4(const GemmArgs& a, int first, int end, int* rows) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int id = first + i < end ? sorted_id(a, first + i) : a.num_tokens;
+    const int tok = id_token(id), slot = id_slot(id);
+    const bool valid = tok < a.num_tokens && slot < a.topk;
+    rows[i] = !valid ? 0
+            : a.a_layout == FLYMOE_ROWS_BY_TOKEN ? tok
+            : a.a_layout == FLYMOE_ROWS_BY_SLOT ? slot * a.num_tokens + tok : tok * a.topk + slot;
+  }
 }
 __device__ __forceinline__ void tcgen05_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -210,6 +248,56 @@ __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wa
 __device__ __forceinline__ void red_add_v4_f32(float* p, float a, float b, float c, float d) {
   asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a), "f"(b), "f"(c), "f"(d) : "memory");
 }
+// ------------------------------------------------------------------------------ clusters
+__device__ __forceinline__ uint32_t cluster_rank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync_all() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void mbar_arrive_rank(uint32_t bar, uint32_t rank) {
+  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(map_to_rank(bar, rank)) : "memory");
+}
+__device__ __forceinline__ uint4 ld_cluster_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+// Wait whose success also orders the other ranks' shared-memory writes (acquire at cluster scope).
+__device__ __forceinline__ uint32_t mbar_try_wait_cluster(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done;
+}
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
+                                                  int code) {
+  if (mbar_try_wait_cluster(bar, parity)) return true;
+  const unsigned long long t0 = global_timer_ns();
+#pragma unroll 1
+  for (uint32_t it = 1;; ++it) {
+    if (mbar_try_wait_cluster(bar, parity)) return true;
+    if ((it & 0xFF) == 0) {
+      if (*abort_flag) return false;
+      if (global_timer_ns() - t0 > kWaitLimitNs) {
+        *abort_flag = 1;
+        atomicCAS(status, 0, code);
+        return false;
+      }
+    }
+  }
+}
 // ------------------------------------------------------------------------------ tiles
 struct TileSched {
   int num_mblocks, num_ntiles, total, group_m;
@@ -224,10 +312,13 @@ struct TileSched {
 };
 
 // ------------------------------------------------------------------------------ host
-int make_gemm_maps(int stage, const GemmArgs& a, CUtensorMap* map_a, CUtensorMap* map_b);
+// Tensor maps of both operands: boxes of `a_box_rows` rows of A and of `b_box_rows` weight rows, 128 bytes of K wide.
+int make_gemm_maps(int stage, const GemmArgs& a, int a_box_rows, int b_box_rows, CUtensorMap* map_a, CUtensorMap* map_b);
 // How many CTAs (one cluster) share a tile's K range; 1 = the one-CTA-per-tile kernel.
 int plan_ksplit(int stage, const GemmArgs& a, int ctas);
 int launch_gemm_split(int stage, const GemmArgs& a, const CUtensorMap& map_a, const CUtensorMap& map_b, int group_m,
                       int split, cudaStream_t stream);
+bool use_pair_kernel(const GemmArgs& a);
+int launch_gemm_pair(int stage, const GemmArgs& a, int ctas, cudaStream_t stream);
 
 }  // namespace flymoe

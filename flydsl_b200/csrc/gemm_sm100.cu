@@ -780,18 +780,16 @@ static int make_map(CUtensorMap* map, const void* base, int rank, const cuuint64
   return FLYMOE_OK;
 }
 
-// Tensor maps of both operands: boxes of tile_m rows of A, and of 128 (stage 1: gate and up rows apart) or
-// 256 weight rows, each 128 bytes of K wide.
-int make_gemm_maps(int stage, const GemmArgs& a, CUtensorMap* map_a, CUtensorMap* map_b) {
+int make_gemm_maps(int stage, const GemmArgs& a, int a_box_rows, int b_box_rows, CUtensorMap* map_a, CUtensorMap* map_b) {
   const long long wrows = stage == 1 ? 2LL * a.n_dim : a.n_dim;
   cuuint64_t adims[2] = {cuuint64_t(a.k_dim), cuuint64_t(a.a_rows)};
   cuuint64_t astrides[1] = {cuuint64_t(a.k_dim)};
-  cuuint32_t abox[2] = {cuuint32_t(BK), cuuint32_t(a.tile_m)};
+  cuuint32_t abox[2] = {cuuint32_t(BK), cuuint32_t(a_box_rows)};
   const int rc = make_map(map_a, a.a, 2, adims, astrides, abox);
   if (rc != FLYMOE_OK) return rc;
   cuuint64_t bdims[3] = {cuuint64_t(a.k_dim), cuuint64_t(wrows), cuuint64_t(a.experts)};
   cuuint64_t bstrides[2] = {cuuint64_t(a.k_dim), cuuint64_t(wrows) * cuuint64_t(a.k_dim)};
-  cuuint32_t bbox[3] = {cuuint32_t(BK), cuuint32_t(stage == 1 ? 128 : BN), 1};
+  cuuint32_t bbox[3] = {cuuint32_t(BK), cuuint32_t(b_box_rows), 1};
   return make_map(map_b, a.w, 3, bdims, bstrides, bbox);
 }
 
@@ -829,18 +827,23 @@ int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {
     set_last_error_msg("tcgen05 GEMM: per-token scaling supports neither per-row destinations nor e4m3 output");
     return FLYMOE_ERR_UNSUPPORTED;
   }
+  const bool limited = g_cta_limit > 0 && g_cta_limit < sm_count();
+  const int ctas = limited ? g_cta_limit : sm_count();
+  if (ctas >= 2 && use_pair_kernel(a)) return launch_gemm_pair(stage, a, ctas, stream);
   CUtensorMap map_a, map_b;
-  int rc = make_gemm_maps(stage, a, &map_a, &map_b);
+  // rows fetched by index come in boxes of one row; stage 1 fetches gate and up rows apart
+  const int rc = make_gemm_maps(stage, a, a.a_layout == FLYMOE_ROWS_SORTED ? a.tile_m : 1, stage == 1 ? 128 : BN,
+                                &map_a, &map_b);
   if (rc != FLYMOE_OK) return rc;
   const long long pairs = (long long)a.num_tokens * a.topk;
   long long g = (pairs + (long long)a.experts * a.tile_m - 1) / ((long long)a.experts * a.tile_m);
   const int group_m = int(g < 1 ? 1 : (g > 16 ? 16 : g));
+  if (!limited) {
+    const int split = plan_ksplit(stage, a, ctas);
+    if (split > 1) return launch_gemm_split(stage, a, map_a, map_b, group_m, split, stream);
+  }
   const int ntiles = stage == 1 ? a.n_dim / 128 : ceil_div(a.n_dim, BN);
   const long long max_tiles = (long long)a.size_expert_ids * ntiles;
-  int ctas = sm_count();
-  if (g_cta_limit > 0 && g_cta_limit < ctas) ctas = g_cta_limit;
-  else if (const int split = plan_ksplit(stage, a, ctas); split > 1)
-    return launch_gemm_split(stage, a, map_a, map_b, group_m, split, stream);
   const int grid = int(max_tiles < ctas ? max_tiles : ctas);
   if (grid <= 0) return FLYMOE_OK;
   if (per_token)

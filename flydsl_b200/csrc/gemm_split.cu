@@ -17,6 +17,7 @@
 // that no shared memory goes away while a peer may still read it.
 #include <cuda.h>
 #include <atomic>
+#include <type_traits>
 
 #include "common.cuh"
 #include "gemm_args.cuh"
@@ -46,57 +47,12 @@ constexpr size_t kSplitSmem = size_t(kSplitStages) * kSplitStageBytes + size_t(k
                               sizeof(SplitCtrl) + 1024;
 static_assert(kSplitSmem <= 232448, "shared memory budget of one SM exceeded");
 
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void mbar_arrive_rank(uint32_t bar, uint32_t rank) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(map_to_rank(bar, rank)) : "memory");
-}
-__device__ __forceinline__ uint4 ld_cluster_v4(uint32_t addr) {
-  uint4 v;
-  asm volatile("ld.shared::cluster.v4.u32 {%0, %1, %2, %3}, [%4];"
-               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
-  return v;
-}
-// Bounded wait whose success also orders the other ranks' shared-memory writes (acquire at cluster scope).
-__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* status,
-                                                  int code) {
-  const unsigned long long t0 = global_timer_ns();
-#pragma unroll 1
-  for (uint32_t it = 1;; ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done) return true;
-    if ((it & 0xFF) == 0) {
-      if (*abort_flag) return false;
-      if (global_timer_ns() - t0 > kWaitLimitNs) {
-        *abort_flag = 1;
-        atomicCAS(status, 0, code);
-        return false;
-      }
-    }
-  }
-}
 __device__ __forceinline__ void red_add_2x16(void* p, uint32_t lo, uint32_t hi, bool bf) {
   if (bf) asm volatile("red.global.add.noftz.v2.bf16x2 [%0], {%1, %2};" ::"l"(p), "r"(lo), "r"(hi) : "memory");
   else asm volatile("red.global.add.noftz.v2.f16x2 [%0], {%1, %2};" ::"l"(p), "r"(lo), "r"(hi) : "memory");
 }
 
-template <int STAGE, int SCALING, bool GATHER>
+template <int STAGE, int SCALING>
 __global__ void __launch_bounds__(kNumThreads, 1)
 moe_gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                       const GemmArgs a, const int group_m, const int split) {
@@ -113,7 +69,7 @@ moe_gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   const int kb0 = int((long long)KB * rank / split), kb1 = int((long long)KB * (rank + 1) / split);
   const int first_tile = int(blockIdx.x) / split, tile_step = int(gridDim.x) / split;
 
-  const int valid_rows = min(__ldg(a.num_valid_ids), a.size_expert_ids * a.tile_m);
+  const int valid_rows = routed_rows(a);
   TileSched sched;
   sched.num_mblocks = (valid_rows + a.tile_m - 1) / a.tile_m;
   sched.num_ntiles = STAGE == 1 ? a.n_dim / 128 : (a.n_dim + BN - 1) / BN;
@@ -122,7 +78,7 @@ moe_gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 
   if (threadIdx.x == 0) {
     for (int i = 0; i < kSplitStages; ++i) {
-      mbar_init(smem_u32(&ctrl->full[i]), GATHER ? 2 : 1);
+      mbar_init(smem_u32(&ctrl->full[i]), 1);
       mbar_init(smem_u32(&ctrl->empty[i]), 1);
     }
     for (int i = 0; i < kAccStages; ++i) {
@@ -148,131 +104,90 @@ moe_gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   static_assert(128 * 40 + 256 * 232 <= kNumThreads * 168, "setmaxnreg split exceeds the launch allocation");
   if (warp < 4) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
-    if (warp == 0 && lane == 0) {
+    const bool gather = a.a_layout != FLYMOE_ROWS_SORTED;
+    if (warp == 0) {
       // ---------------------------------------------------------------- TMA producer
       int stage = 0;
       uint32_t phase = 0;
-      const uint32_t tx_bytes = (GATHER ? 0u : uint32_t(a.tile_m) * BK) + kBTileBytes;
+      const uint32_t tx_bytes = uint32_t(a.tile_m) * BK + kBTileBytes;
       bool ok = true;
       for (int t = first_tile; t < sched.total && ok; t += tile_step) {
         int mb, n;
         sched.decode(t, mb, n);
-        const int e = __ldg(a.sorted_expert_ids + mb);
+        const int e = block_expert(a, mb);
         if (e < 0 || e >= a.experts) continue;
+        int rows[4];
+        if (gather) gather_rows4(a, mb * a.tile_m + lane * 4, min((mb + 1) * a.tile_m, valid_rows), rows);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(smem_u32(&ctrl->empty[stage]), phase ^ 1, abort_flag, a.status, 1, 64)) { ok = false; break; }
+          ok = warp_wait(smem_u32(&ctrl->empty[stage]), phase ^ 1, abort_flag, a.status, 1, 64);
+          if (!ok) break;
           const uint32_t full = smem_u32(&ctrl->full[stage]);
           const uint32_t sa = smem_u32(smem + size_t(stage) * kSplitStageBytes);
           const uint32_t sb = sa + kSplitAStage;
-          mbar_expect_tx(full, tx_bytes);
-          if (!GATHER) tma_load_2d(sa, &tmap_a, full, kb * BK, mb * a.tile_m);
-          if (STAGE == 1) {
-            tma_load_3d(sb, &tmap_b, full, kb * BK, n * 128, e);
-            tma_load_3d(sb + 128 * BK, &tmap_b, full, kb * BK, a.n_dim + n * 128, e);
-          } else {
-            tma_load_3d(sb, &tmap_b, full, kb * BK, n * BN, e);
-          }
-          if (++stage == kSplitStages) { stage = 0; phase ^= 1; }
-        }
-      }
-    } else if (warp == 1 && lane == 0) {
-      // ---------------------------------------------------------------- MMA issuer
-      int stage = 0, acc = 0;
-      uint32_t phase = 0, acc_phase = 0;
-      bool ok = true;
-      const bool int8_ops = SCALING == kScalePerToken && a.in_dtype == FLYMOE_I8;
-      const bool half_ops = SCALING == kScalePerToken && (a.in_dtype == FLYMOE_F16 || a.in_dtype == FLYMOE_BF16);
-      const uint32_t half_desc = a.in_dtype == FLYMOE_BF16 ? kInstrDescBF16 : kInstrDescF16;
-      for (int t = first_tile; t < sched.total && ok; t += tile_step) {
-        int mb, n;
-        sched.decode(t, mb, n);
-        const int e = __ldg(a.sorted_expert_ids + mb);
-        if (e < 0 || e >= a.experts) continue;
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (SCALING == kScaleBlock128 || kb == kb0) {
-            if (!mbar_wait(smem_u32(&ctrl->tmem_empty[acc]), acc_phase ^ 1, abort_flag, a.status, 2)) { ok = false; break; }
-          }
-          if (!mbar_wait(smem_u32(&ctrl->full[stage]), phase, abort_flag, a.status, 3)) { ok = false; break; }
-          tcgen05_fence_after();
-          const uint32_t sa = smem_u32(smem + size_t(stage) * kSplitStageBytes);
-          const uint64_t adesc = make_smem_desc(sa);
-          const uint64_t bdesc = make_smem_desc(sa + kSplitAStage);
-          const uint32_t d_tmem = tmem_base + uint32_t(acc) * BN;
-#pragma unroll
-          for (int k = 0; k < BK / 32; ++k) {
-            const uint32_t accumulate = (k > 0 || (SCALING == kScalePerToken && kb > kb0)) ? 1u : 0u;
-            if (int8_ops) umma_i8(d_tmem, adesc + uint64_t(k * 2), bdesc + uint64_t(k * 2), kInstrDescI8, accumulate);
-            else if (half_ops) umma_f16(d_tmem, adesc + uint64_t(k * 2), bdesc + uint64_t(k * 2), half_desc, accumulate);
-            else umma_f8(d_tmem, adesc + uint64_t(k * 2), bdesc + uint64_t(k * 2), kInstrDescF8, accumulate);
-          }
-          umma_commit(smem_u32(&ctrl->empty[stage]));
-          if (SCALING == kScaleBlock128 || kb + 1 == kb1) {
-            umma_commit(smem_u32(&ctrl->tmem_full[acc]));
-            if (++acc == kAccStages) { acc = 0; acc_phase ^= 1; }
-          }
-          if (++stage == kSplitStages) { stage = 0; phase ^= 1; }
-        }
-      }
-    } else if (warp == 3 && GATHER) {
-      // ---------------------------------------------------------------- row gather (see gemm_sm100.cu)
-      constexpr int kInFlight = 2;
-      int stage = 0, pending = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      const int pad_id = (a.topk << 24) | a.num_tokens;
-      auto complete_oldest = [&]() {
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        __syncwarp();
-        const int s_old = (stage - pending + 2 * kSplitStages) % kSplitStages;
-        if (lane == 0) mbar_arrive(smem_u32(&ctrl->full[s_old]));
-        --pending;
-      };
-      for (int t = first_tile; t < sched.total && ok; t += tile_step) {
-        int mb, n;
-        sched.decode(t, mb, n);
-        const int e = __ldg(a.sorted_expert_ids + mb);
-        if (e < 0 || e >= a.experts) continue;
-        constexpr int kRowsPerLane = kSplitMaxRows / 32;
-        const uint8_t* src[kRowsPerLane];
-        uint32_t nbytes[kRowsPerLane];           // 16 = copy, 0 = zero-fill (pad row)
-#pragma unroll
-        for (int j = 0; j < kRowsPerLane; ++j) {
-          const int row = j * 32 + lane;
-          const int r = mb * a.tile_m + row;
-          const int id = (row < a.tile_m && r < valid_rows) ? __ldg(a.sorted_ids + r) : pad_id;
-          const int tok = id_token(id), slot = id_slot(id);
-          const bool valid = tok < a.num_tokens && slot < a.topk;
-          const long long srow = a.a_layout == FLYMOE_ROWS_BY_TOKEN ? (long long)tok
-                               : a.a_layout == FLYMOE_ROWS_BY_SLOT ? (long long)slot * a.num_tokens + tok
-                                                                   : (long long)tok * a.topk + slot;
-          src[j] = a.a + (valid ? srow : 0) * a.k_dim;
-          nbytes[j] = valid ? 16u : 0u;
-        }
-        for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(smem_u32(&ctrl->empty[stage]), phase ^ 1, abort_flag, a.status, 10, 32)) { ok = false; break; }
-          const uint32_t sa = smem_u32(smem + size_t(stage) * kSplitStageBytes);
-#pragma unroll
-          for (int j = 0; j < kRowsPerLane; ++j) {
-            const int row = j * 32 + lane;
-            if (row < a.tile_m) {
-              const uint8_t* g = src[j] + kb * BK;
-              const uint32_t d = sa + uint32_t(row) * 128u;
-#pragma unroll
-              for (int c = 0; c < 8; ++c)
-                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
-                             ::"r"(d + (uint32_t(c ^ (row & 7)) << 4)), "l"(g + c * 16), "r"(nbytes[j]) : "memory");
+          if (elect_one()) {
+            mbar_expect_tx(full, tx_bytes);
+            if (!gather) tma_load_2d(sa, &tmap_a, full, kb * BK, mb * a.tile_m);
+            if (STAGE == 1) {
+              tma_load_3d(sb, &tmap_b, full, kb * BK, n * 128, e);
+              tma_load_3d(sb + 128 * BK, &tmap_b, full, kb * BK, a.n_dim + n * 128, e);
+            } else {
+              tma_load_3d(sb, &tmap_b, full, kb * BK, n * BN, e);
             }
           }
-          asm volatile("cp.async.commit_group;" ::: "memory");
-          if (++stage == kSplitStages) { stage = 0; phase ^= 1; }
-          if (++pending > kInFlight) {
-            asm volatile("cp.async.wait_group %0;" ::"n"(kInFlight) : "memory");
-            complete_oldest();
+          if (gather) {
+            __syncwarp();                        // the expected byte count is set before any of it can arrive
+            if (lane * 4 < a.tile_m) tma_gather4(sa + uint32_t(lane) * 512u, &tmap_a, full, kb * BK, rows);
           }
+          if (++stage == kSplitStages) { stage = 0; phase ^= 1; }
         }
       }
-      asm volatile("cp.async.wait_group 0;" ::: "memory");
-      while (pending > 0) complete_oldest();
+    } else if (warp == 1) {
+      // ---------------------------------------------------------------- MMA issuer
+      auto issue = [&](auto kind_c, uint32_t idesc) {
+        constexpr int KIND = decltype(kind_c)::value;
+        int stage = 0, acc = 0;
+        uint32_t phase = 0, acc_phase = 0;
+        int mb = 0, n = 0, e_next = -1;                    // expert id: loaded a whole tile early
+        if (int(first_tile) < sched.total) {
+          sched.decode(first_tile, mb, n);
+          e_next = block_expert(a, mb);
+        }
+        for (int t = first_tile; t < sched.total; t += tile_step) {
+          const int e = e_next;
+          if (t + int(tile_step) < sched.total) {
+            sched.decode(t + tile_step, mb, n);
+            e_next = block_expert(a, mb);
+          }
+          if (e < 0 || e >= a.experts) continue;
+          for (int kb = kb0; kb < kb1; ++kb) {
+            // per-token scaling: one accumulator stage per tile; block scaling: one per K block, started from zero
+            if (SCALING == kScaleBlock128 || kb == kb0) {
+              if (!warp_wait(smem_u32(&ctrl->tmem_empty[acc]), acc_phase ^ 1, abort_flag, a.status, 2)) return;
+            }
+            if (!warp_wait(smem_u32(&ctrl->full[stage]), phase, abort_flag, a.status, 3)) return;
+            tcgen05_fence_after();
+            const uint32_t sa = smem_u32(smem + size_t(stage) * kSplitStageBytes);
+            const uint64_t adesc = make_smem_desc(sa);
+            const uint64_t bdesc = make_smem_desc(sa + kSplitAStage);
+            const uint32_t d_tmem = tmem_base + uint32_t(acc) * BN;
+            const bool last = SCALING == kScaleBlock128 || kb + 1 == kb1;
+            if (elect_one()) {
+#pragma unroll
+              for (int k = 0; k < BK / 32; ++k)
+                umma<KIND>(d_tmem, adesc + uint64_t(k * 2), bdesc + uint64_t(k * 2), idesc,
+                           (k > 0 || (SCALING == kScalePerToken && kb > kb0)) ? 1u : 0u);
+              umma_commit(smem_u32(&ctrl->empty[stage]));
+              if (last) umma_commit(smem_u32(&ctrl->tmem_full[acc]));
+            }
+            __syncwarp();
+            if (last && ++acc == kAccStages) { acc = 0; acc_phase ^= 1; }
+            if (++stage == kSplitStages) { stage = 0; phase ^= 1; }
+          }
+        }
+      };
+      if (SCALING == kScaleBlock128 || a.in_dtype == FLYMOE_E4M3) issue(std::integral_constant<int, 0>{}, kInstrDescF8);
+      else if (a.in_dtype == FLYMOE_I8) issue(std::integral_constant<int, 1>{}, kInstrDescI8);
+      else issue(std::integral_constant<int, 2>{}, a.in_dtype == FLYMOE_BF16 ? kInstrDescBF16 : kInstrDescF16);
     }
     __syncwarp();
   } else {
@@ -295,7 +210,7 @@ moe_gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     for (int t = first_tile; t < sched.total && ok; t += tile_step) {
       int mb, n;
       sched.decode(t, mb, n);
-      const int e = __ldg(a.sorted_expert_ids + mb);
+      const int e = block_expert(a, mb);
       if (e < 0 || e >= a.experts) continue;
       // index of a row's activation scale, -1 for pad rows
       auto scale_row = [&](int r, int id) -> long long {
@@ -308,7 +223,7 @@ moe_gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       };
       auto row_id = [&](int row) {
         const int r = mb * a.tile_m + row;
-        return (row < a.tile_m && r < valid_rows) ? __ldg(a.sorted_ids + r) : pad_id;
+        return (row < a.tile_m && r < valid_rows) ? sorted_id(a, r) : pad_id;
       };
       // ---- this rank's K blocks --------------------------------------------------------
       const bool half_ok = STAGE == 1 ? true : (n * BN + wg * 128 < a.n_dim);
@@ -522,10 +437,10 @@ moe_gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 }
 
 // ------------------------------------------------------------------------------ host
-template <int STAGE, int SCALING, bool GATHER>
+template <int STAGE, int SCALING>
 static int launch_split(const GemmArgs& a, const CUtensorMap& map_a, const CUtensorMap& map_b, int group_m, int split,
                         cudaStream_t stream) {
-  auto* kernel = moe_gemm_split_kernel<STAGE, SCALING, GATHER>;
+  auto* kernel = moe_gemm_split_kernel<STAGE, SCALING>;
   FLYMOE_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSplitSmem)));
   cudaLaunchAttribute attr;
   attr.id = cudaLaunchAttributeClusterDimension;
@@ -556,21 +471,13 @@ static int launch_split(const GemmArgs& a, const CUtensorMap& map_a, const CUten
   return FLYMOE_OK;
 }
 
-template <int STAGE, int SCALING>
-static int launch_split_rows(const GemmArgs& a, const CUtensorMap& map_a, const CUtensorMap& map_b, int group_m,
-                             int split, cudaStream_t stream) {
-  if (a.a_layout != FLYMOE_ROWS_SORTED)
-    return launch_split<STAGE, SCALING, true>(a, map_a, map_b, group_m, split, stream);
-  return launch_split<STAGE, SCALING, false>(a, map_a, map_b, group_m, split, stream);
-}
-
 int launch_gemm_split(int stage, const GemmArgs& a, const CUtensorMap& map_a, const CUtensorMap& map_b, int group_m,
                       int split, cudaStream_t stream) {
   if (a.scaling == FLYMOE_SCALE_PER_TOKEN)
-    return stage == 1 ? launch_split_rows<1, kScalePerToken>(a, map_a, map_b, group_m, split, stream)
-                      : launch_split_rows<2, kScalePerToken>(a, map_a, map_b, group_m, split, stream);
-  return stage == 1 ? launch_split_rows<1, kScaleBlock128>(a, map_a, map_b, group_m, split, stream)
-                    : launch_split_rows<2, kScaleBlock128>(a, map_a, map_b, group_m, split, stream);
+    return stage == 1 ? launch_split<1, kScalePerToken>(a, map_a, map_b, group_m, split, stream)
+                      : launch_split<2, kScalePerToken>(a, map_a, map_b, group_m, split, stream);
+  return stage == 1 ? launch_split<1, kScaleBlock128>(a, map_a, map_b, group_m, split, stream)
+                    : launch_split<2, kScaleBlock128>(a, map_a, map_b, group_m, split, stream);
 }
 
 int plan_ksplit(int stage, const GemmArgs& a, int ctas) {
