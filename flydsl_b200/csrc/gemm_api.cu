@@ -277,10 +277,6 @@ extern "C" int flymoe_blockscale_gemm(void* c, const void* a, const float* scale
   int* sorted_expert_ids = workspace + rows_padded;
   int* num_valid_ids = sorted_expert_ids + blocks;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  dense_routing_kernel<<<(rows_padded + 255) / 256, 256, 0, s>>>(sorted_ids, sorted_expert_ids, num_valid_ids, m,
-                                                                 rows_padded, blocks);
-  FLYMOE_CUDA_CHECK(cudaGetLastError());
-
   GemmArgs g;
   g.a = static_cast<const uint8_t*>(a);
   g.scale_a = scale_a;
@@ -291,10 +287,8 @@ extern "C" int flymoe_blockscale_gemm(void* c, const void* a, const float* scale
   g.a_rows = m;                       // rows beyond M are filled with zeros by the TMA unit, never read from memory
   g.w = static_cast<const uint8_t*>(b);
   g.scale_w = scale_b;
-  g.sorted_ids = sorted_ids;
-  g.sorted_expert_ids = sorted_expert_ids;
+  g.sorted_ids = g.sorted_expert_ids = g.num_valid_ids = nullptr;
   g.sorted_weights = nullptr;
-  g.num_valid_ids = num_valid_ids;
   g.out = c;
   g.out_scale = nullptr;
   g.out_scale_stride = 0;
@@ -313,5 +307,17 @@ extern "C" int flymoe_blockscale_gemm(void* c, const void* a, const float* scale
   g.size_expert_ids = blocks;
   g.tile_m = tile_m;
   g.status = status;
+  // Identity routing: the cluster kernel computes it (null tables), which saves a launch where launches count
+  // (M=64 N=2112 K=7168: 18.4 -> 14.5 us a call).  The one-CTA kernel reads
+  // tables: looking up its routing conditionally cost the M=4096 case 3.6 %.
+  g.ksplit = choose_ksplit(2, g);
+  if (g.ksplit <= 1) {
+    dense_routing_kernel<<<(rows_padded + 255) / 256, 256, 0, s>>>(sorted_ids, sorted_expert_ids, num_valid_ids, m,
+                                                                   rows_padded, blocks);
+    FLYMOE_CUDA_CHECK(cudaGetLastError());
+    g.sorted_ids = sorted_ids;
+    g.sorted_expert_ids = sorted_expert_ids;
+    g.num_valid_ids = num_valid_ids;
+  }
   return launch_gemm_sm100(2, g, s);
 }

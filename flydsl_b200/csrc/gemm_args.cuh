@@ -41,10 +41,13 @@ struct GemmArgs {
   int n_dim;                   // stage 1: inter_dim; stage 2: model_dim
   int k_dim;                   // stage 1: model_dim; stage 2: inter_dim
   int size_expert_ids, tile_m;
+  int ksplit = 0;              // CTAs per tile, decided by the entry point; 0 = decide at launch
   int* status;                 // device status word (bounded waits report here)
 };
 
 int launch_gemm_simt(int stage, const GemmArgs& args, cudaStream_t stream);
 int launch_gemm_sm100(int stage, const GemmArgs& args, cudaStream_t stream);
+// CTAs that launch_gemm_sm100 would give one tile (1: the one-CTA-per-tile kernels).
+int choose_ksplit(int stage, const GemmArgs& args);
 
 }  // namespace flymoe

@@ -100,7 +100,7 @@ __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
       ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2) : "memory");
 }
-// Routing of the launch.  A null sorted_ids is the identity routing of the dense GEMM: sorted row r is row r, every
+// Routing of the cluster kernel.  Null sorted_ids: identity routing of the dense GEMM -- sorted row r is row r, every
 // row block belongs to expert 0, and all row blocks are in use -- no tables to write first.
 __device__ __forceinline__ int routed_rows(const GemmArgs& a) {
   const int cap = a.size_expert_ids * a.tile_m;

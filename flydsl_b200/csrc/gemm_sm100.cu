@@ -812,6 +812,12 @@ static int launch_one(int grid, cudaStream_t stream, const CUtensorMap& map_a, c
   return launch_kernel<STAGE, ROW_DST, SCALING, false>(grid, stream, map_a, map_b, a, group_m);
 }
 
+int choose_ksplit(int stage, const GemmArgs& a) {
+  // a caller that leaves other kernels some SMs gets no clusters
+  if (g_cta_limit > 0 && g_cta_limit < sm_count()) return 1;
+  return plan_ksplit(stage, a, sm_count());
+}
+
 int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {
   if (a.tile_m != 16 && a.tile_m != 32 && a.tile_m != 64 && a.tile_m != 128) {
     set_last_error_msg("tcgen05 GEMM: tile_m must be 16, 32, 64 or 128");
@@ -827,8 +833,7 @@ int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {
     set_last_error_msg("tcgen05 GEMM: per-token scaling supports neither per-row destinations nor e4m3 output");
     return FLYMOE_ERR_UNSUPPORTED;
   }
-  const bool limited = g_cta_limit > 0 && g_cta_limit < sm_count();
-  const int ctas = limited ? g_cta_limit : sm_count();
+  const int ctas = g_cta_limit > 0 && g_cta_limit < sm_count() ? g_cta_limit : sm_count();
   if (ctas >= 2 && use_pair_kernel(a)) return launch_gemm_pair(stage, a, ctas, stream);
   CUtensorMap map_a, map_b;
   // rows fetched by index come in boxes of one row; stage 1 fetches gate and up rows apart
@@ -838,10 +843,8 @@ int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {
   const long long pairs = (long long)a.num_tokens * a.topk;
   long long g = (pairs + (long long)a.experts * a.tile_m - 1) / ((long long)a.experts * a.tile_m);
   const int group_m = int(g < 1 ? 1 : (g > 16 ? 16 : g));
-  if (!limited) {
-    const int split = plan_ksplit(stage, a, ctas);
-    if (split > 1) return launch_gemm_split(stage, a, map_a, map_b, group_m, split, stream);
-  }
+  const int split = a.ksplit > 0 ? a.ksplit : choose_ksplit(stage, a);
+  if (split > 1) return launch_gemm_split(stage, a, map_a, map_b, group_m, split, stream);
   const int ntiles = stage == 1 ? a.n_dim / 128 : ceil_div(a.n_dim, BN);
   const long long max_tiles = (long long)a.size_expert_ids * ntiles;
   const int grid = int(max_tiles < ctas ? max_tiles : ctas);
