@@ -6,8 +6,11 @@
 // gives every warp its write cursor per expert, and a warp-level match gives each
 // pair its rank inside a 32-pair step, so the scatter is deterministic.
 //   * P <= kOneBlockMaxPairs : one launch, one block, everything in shared memory.
-//   * otherwise              : count (grid) -> scan (one block) -> scatter (grid),
-//                              per-segment histograms kept in caller-provided scratch.
+//   * otherwise              : count (grid) -> scan (one block) -> scatter (grid).  Only the totals of
+//                              a block's eight segments go through caller-provided scratch; the
+//                              scatter kernel counts its own segments again (a few loads per lane),
+//                              which makes the one-block scan, the serial part, eight times shorter.
+// The caller's accumulation buffer is cleared by extra blocks of the first launch, beside the sort.
 #include <stdio.h>
 
 #include "common.cuh"
@@ -28,8 +31,11 @@ struct SortArgs {
   int* sorted_expert_ids;
   int* num_valid_ids;
   const int* expert_mask;
-  int* ws_counts;   // [nseg][E] on the multi-block path
+  int* ws_counts;   // [nblk][E] on the multi-block path: totals per block, then their exclusive prefix
   int* ws_base;     // [E]
+  uint8_t* zero_buf;            // cleared by the blocks behind the first `sort_blocks` ones
+  long long zero_bytes;
+  int sort_blocks, nblk;
   int num_tokens, num_experts, topk, unit_size;
   int num_pairs, seg_len, nseg;
   int sorted_capacity, expert_ids_capacity;
@@ -146,7 +152,21 @@ __device__ void block_layout(const SortArgs& a, const int* tot, int* base, int* 
   }
 }
 
+// Clears this block's share of the accumulation buffer: 16-byte stores between the aligned ends.
+__device__ __forceinline__ void clear_share(const SortArgs& a) {
+  const int nb = gridDim.x - a.sort_blocks, b = blockIdx.x - a.sort_blocks;
+  uint8_t* p = a.zero_buf;
+  const long long head = min((long long)((16 - (reinterpret_cast<uintptr_t>(p) & 15)) & 15), a.zero_bytes);
+  const long long nvec = (a.zero_bytes - head) / 16;
+  const long long i0 = (long long)b * blockDim.x + threadIdx.x, step = (long long)nb * blockDim.x;
+  uint4* v = reinterpret_cast<uint4*>(p + head);
+  for (long long i = i0; i < nvec; i += step) v[i] = make_uint4(0, 0, 0, 0);
+  for (long long i = i0; i < head; i += step) p[i] = 0;
+  for (long long i = head + nvec * 16 + i0; i < a.zero_bytes; i += step) p[i] = 0;
+}
+
 __global__ void __launch_bounds__(kSortThreads) moe_sort_oneblock_kernel(SortArgs a) {
+  if (int(blockIdx.x) >= a.sort_blocks) { clear_share(a); return; }
   extern __shared__ int smem[];
   const int E = a.num_experts;
   int* cnt = smem;                       // [kSortWarps][E]
@@ -174,25 +194,31 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_oneblock_kernel(SortArg
   warp_scatter(a, warp, cnt + warp * E, base, lane);
 }
 
-// Multi-block path, step 1: per-segment histograms to scratch.
-__global__ void __launch_bounds__(kSortThreads) moe_sort_count_kernel(SortArgs a) {
-  extern __shared__ int smem[];
-  const int E = a.num_experts;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int* cnt = smem + warp * E;
-  for (int i = tid; i < kSortWarps * E; i += kSortThreads) smem[i] = 0;
+// Histograms of this block's eight segments into smem [kSortWarps][E].
+__device__ __forceinline__ void block_count(const SortArgs& a, int* cnt) {
+  for (int i = threadIdx.x; i < kSortWarps * a.num_experts; i += kSortThreads) cnt[i] = 0;
   __syncthreads();
-  const int seg = blockIdx.x * kSortWarps + warp;
-  if (seg < a.nseg) {
-    warp_count(a, seg, cnt, lane);
-    __syncwarp();
-    for (int e = lane; e < E; e += 32) a.ws_counts[size_t(seg) * E + e] = cnt[e];
+  const int warp = threadIdx.x >> 5, seg = blockIdx.x * kSortWarps + warp;
+  if (seg < a.nseg) warp_count(a, seg, cnt + warp * a.num_experts, threadIdx.x & 31);
+  __syncthreads();
+}
+
+// Multi-block path, step 1: block totals to scratch.
+__global__ void __launch_bounds__(kSortThreads) moe_sort_count_kernel(SortArgs a) {
+  if (int(blockIdx.x) >= a.sort_blocks) { clear_share(a); return; }
+  extern __shared__ int smem[];
+  block_count(a, smem);
+  for (int e = threadIdx.x; e < a.num_experts; e += kSortThreads) {
+    int sum = 0;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) sum += smem[w * a.num_experts + e];
+    a.ws_counts[size_t(blockIdx.x) * a.num_experts + e] = sum;
   }
 }
 
-// Step 2 (one block of 1024 threads): exclusive prefix over segments per expert, then the expert
-// layout.  The segment axis is cut into `parts` contiguous ranges handled by different threads of
-// the same expert (parts * E <= 1024), so the serial walk per thread is nseg / parts long.
+// Step 2 (one block of 1024 threads): exclusive prefix over blocks per expert, then the expert
+// layout.  The block axis is cut into `parts` contiguous ranges handled by different threads of
+// the same expert (parts * E <= 1024), so the serial walk per thread is nblk / parts long.
 __global__ void __launch_bounds__(1024) moe_sort_scan_kernel(SortArgs a) {
   __shared__ int tot[kMaxExperts];
   __shared__ int base[kMaxExperts];
@@ -200,11 +226,11 @@ __global__ void __launch_bounds__(1024) moe_sort_scan_kernel(SortArgs a) {
   __shared__ int part_sum[1024];
   const int E = a.num_experts;
   int parts = 1;
-  while (parts * 2 * E <= 1024 && parts * 2 <= a.nseg) parts *= 2;
-  const int per_part = (a.nseg + parts - 1) / parts;
+  while (parts * 2 * E <= 1024 && parts * 2 <= a.nblk) parts *= 2;
+  const int per_part = (a.nblk + parts - 1) / parts;
   const int e = threadIdx.x % E, part = threadIdx.x / E;
   const bool active = part < parts && threadIdx.x < parts * E;
-  const int s0 = min(part * per_part, a.nseg), s1 = min(s0 + per_part, a.nseg);
+  const int s0 = min(part * per_part, a.nblk), s1 = min(s0 + per_part, a.nblk);
   int sum = 0;
   if (active) {
 #pragma unroll 8
@@ -233,15 +259,22 @@ __global__ void __launch_bounds__(kSortThreads) moe_sort_scatter_kernel(SortArgs
   extern __shared__ int smem[];
   const int E = a.num_experts;
   int* base = smem;                      // [E]
-  int* cur_all = smem + E;               // [kSortWarps][E]
+  int* cur = smem + E;                   // [kSortWarps][E]
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int e = tid; e < E; e += kSortThreads) base[e] = a.ws_base[e];
-  const int seg = blockIdx.x * kSortWarps + warp;
-  int* cur = cur_all + warp * E;
-  if (seg < a.nseg)
-    for (int e = lane; e < E; e += 32) cur[e] = a.ws_counts[size_t(seg) * E + e];
+  block_count(a, cur);
+  for (int e = tid; e < E; e += kSortThreads) {      // write cursors: blocks before, then the warps before
+    base[e] = a.ws_base[e];
+    int run = a.ws_counts[size_t(blockIdx.x) * E + e];
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) {
+      const int c = cur[w * E + e];
+      cur[w * E + e] = run;
+      run += c;
+    }
+  }
   __syncthreads();
-  if (seg < a.nseg) warp_scatter(a, seg, cur, base, lane);
+  const int seg = blockIdx.x * kSortWarps + warp;
+  if (seg < a.nseg) warp_scatter(a, seg, cur + warp * E, base, lane);
 }
 
 static void sort_plan(int num_pairs, int* seg_len, int* nseg, bool* one_block) {
@@ -306,15 +339,22 @@ extern "C" int flymoe_moe_sorting(const int32_t* topk_ids, const float* topk_wei
   sort_plan(a.num_pairs, &a.seg_len, &a.nseg, &one_block);
   a.ws_counts = nullptr; a.ws_base = nullptr;
 
-  if (moe_buf != nullptr && moe_buf_bytes > 0)
-    FLYMOE_CUDA_CHECK(cudaMemsetAsync(moe_buf, 0, size_t(moe_buf_bytes), s));
+  // blocks that clear the accumulation buffer: 16 KB each, at most two waves of small blocks
+  a.zero_buf = static_cast<uint8_t*>(moe_buf);
+  a.zero_bytes = moe_buf != nullptr && moe_buf_bytes > 0 ? moe_buf_bytes : 0;
+  int zero_blocks = 0;
+  if (a.zero_bytes > 0) {
+    const long long want = (a.zero_bytes + 16383) / 16384, most = 8LL * sm_count();
+    zero_blocks = int(want < most ? want : (most > 0 ? most : 1));
+  }
 
   if (one_block) {
     const size_t smem = size_t(kSortWarps + 2) * num_experts * sizeof(int) + 64 * sizeof(int);
     if (smem > 48 * 1024)
       FLYMOE_CUDA_CHECK(cudaFuncSetAttribute(moe_sort_oneblock_kernel,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    moe_sort_oneblock_kernel<<<1, kSortThreads, smem, s>>>(a);
+    a.sort_blocks = a.nblk = 1;
+    moe_sort_oneblock_kernel<<<1 + zero_blocks, kSortThreads, smem, s>>>(a);
     FLYMOE_CUDA_CHECK(cudaGetLastError());
     return FLYMOE_OK;
   }
@@ -327,12 +367,13 @@ extern "C" int flymoe_moe_sorting(const int32_t* topk_ids, const float* topk_wei
   a.ws_counts = workspace;
   a.ws_base = workspace + int64_t(a.nseg) * num_experts;
   const int nblk = ceil_div(a.nseg, kSortWarps);
+  a.sort_blocks = a.nblk = nblk;
   const size_t smem_cnt = size_t(kSortWarps) * num_experts * sizeof(int);
   const size_t smem_sct = size_t(kSortWarps + 1) * num_experts * sizeof(int);
   if (smem_sct > 48 * 1024)
     FLYMOE_CUDA_CHECK(cudaFuncSetAttribute(moe_sort_scatter_kernel,
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_sct)));
-  moe_sort_count_kernel<<<nblk, kSortThreads, smem_cnt, s>>>(a);
+  moe_sort_count_kernel<<<nblk + zero_blocks, kSortThreads, smem_cnt, s>>>(a);
   FLYMOE_CUDA_CHECK(cudaGetLastError());
   moe_sort_scan_kernel<<<1, 1024, 0, s>>>(a);
   FLYMOE_CUDA_CHECK(cudaGetLastError());
