@@ -36,7 +36,6 @@ namespace flymoe {
 constexpr int kPairThreads = 640;
 constexpr int kPairEpiWarps = 16;
 constexpr int kPairStageBytes = kATileBytes + kBTileBytes / 2;      // 32 KB per CTA and K block
-constexpr int kPairTable = 4096;                                    // row blocks the tile table covers
 template <int STAGE> struct PairCfg {
   static constexpr int ring = STAGE == 1 ? 6 : 4;
   // stage 2: finished output rows, 256 16-bit results; 16 bytes of skew against bank conflicts
@@ -53,9 +52,8 @@ struct __align__(16) PairCtrl {
   unsigned long long stg_dst[BM];
   uint32_t tmem_base;
   int abort_flag;
-  int num_tiles;
   int scan[2][32];
-  uint16_t table[kPairTable];                   // row tile -> first row block | (row blocks - 1) << 12
+  uint16_t table[kTileTable];                   // see build_tile_table
 };
 template <int STAGE> constexpr size_t pair_smem() {
   return size_t(PairCfg<STAGE>::ring) * kPairStageBytes + size_t(BM) * PairCfg<STAGE>::pitch + sizeof(PairCtrl) + 1024;
@@ -98,30 +96,6 @@ __device__ __forceinline__ void umma_commit_pair(uint32_t bar) {
                ::"r"(bar), "h"(uint16_t(3)) : "memory");
 }
 
-// Block-wide exclusive scan over kPairThreads threads (20 warps): running maximum, then running sum.
-template <bool MAX>
-__device__ __forceinline__ int block_scan_excl(int v, int* scratch, int* total) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  constexpr int kWarps = kPairThreads / 32;
-  int inc = v;
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const int o = __shfl_up_sync(0xffffffffu, inc, off);
-    if (lane >= off) inc = MAX ? max(inc, o) : inc + o;
-  }
-  if (lane == 31) scratch[warp] = inc;
-  __syncthreads();
-  int before = MAX ? -1 : 0, all = MAX ? -1 : 0;
-  for (int w = 0; w < kWarps; ++w) {
-    if (w == warp) before = all;
-    all = MAX ? max(all, scratch[w]) : all + scratch[w];
-  }
-  const int prev = __shfl_up_sync(0xffffffffu, inc, 1);
-  *total = all;
-  if (lane == 0) return before;
-  return MAX ? max(before, prev) : before + prev;
-}
-
 template <int STAGE>
 __global__ void __launch_bounds__(kPairThreads, 1)
 moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
@@ -160,37 +134,7 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
                  ::"r"(smem_u32(&ctrl->tmem_base)), "r"(uint32_t(kTmemCols)) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
-  {
-    // Tile table: within an expert's run of row blocks, every (256 / tile_m)-th block starts a tile.
-    const int nblk = min((valid_rows + a.tile_m - 1) / a.tile_m, kPairTable);
-    const int bpt = 2 * BM / a.tile_m;                           // row blocks per tile: 2 or 4
-    const int per = (nblk + kPairThreads - 1) / kPairThreads;
-    const int b0 = min(int(threadIdx.x) * per, nblk), b1 = min(b0 + per, nblk);
-    int run = -1;                                                // last run start inside this thread's blocks
-    for (int b = b0; b < b1; ++b)
-      if (b == 0 || __ldg(a.sorted_expert_ids + b) != __ldg(a.sorted_expert_ids + b - 1)) run = b;
-    int unused, total;
-    const int run_before = block_scan_excl<true>(run, ctrl->scan[0], &unused);
-    int starts = 0;
-    run = run_before;
-    for (int b = b0; b < b1; ++b) {
-      const int e = __ldg(a.sorted_expert_ids + b);
-      if (b == 0 || e != __ldg(a.sorted_expert_ids + b - 1)) run = b;
-      if (((b - run) & (bpt - 1)) == 0 && e >= 0 && e < a.experts) ++starts;
-    }
-    int at = block_scan_excl<false>(starts, ctrl->scan[1], &total);
-    run = run_before;
-    for (int b = b0; b < b1; ++b) {
-      const int e = __ldg(a.sorted_expert_ids + b);
-      if (b == 0 || e != __ldg(a.sorted_expert_ids + b - 1)) run = b;
-      if (((b - run) & (bpt - 1)) == 0 && e >= 0 && e < a.experts) {
-        int nb = 1;
-        while (nb < bpt && b + nb < nblk && __ldg(a.sorted_expert_ids + b + nb) == e) ++nb;
-        ctrl->table[at++] = uint16_t(b | ((nb - 1) << 12));
-      }
-    }
-    if (threadIdx.x == 0) ctrl->num_tiles = total;
-  }
+  const int num_tiles = build_tile_table<kPairThreads>(a, valid_rows, 2 * BM / a.tile_m, ctrl->table, ctrl->scan);
   tcgen05_fence_before();
   __syncthreads();
   cluster_sync_all();                            // both CTAs' barriers and TMEM exist
@@ -198,7 +142,7 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   const uint32_t tmem_base = ctrl->tmem_base;
 
   TileSched sched;
-  sched.num_mblocks = ctrl->num_tiles;
+  sched.num_mblocks = num_tiles;
   sched.num_ntiles = STAGE == 1 ? a.n_dim / 128 : (a.n_dim + BN - 1) / BN;
   sched.total = sched.num_mblocks * sched.num_ntiles;
   sched.group_m = group_m;
@@ -491,7 +435,7 @@ static int launch_pair(const GemmArgs& a, const CUtensorMap& map_a, const CUtens
 // blocks) 1044 against 1179.
 bool use_pair_kernel(const GemmArgs& a) {
   if (a.scaling != FLYMOE_SCALE_PER_TOKEN || a.tile_m < 64 || a.a_layout != FLYMOE_ROWS_SORTED) return false;
-  if (a.size_expert_ids > kPairTable) return false;
+  if (a.size_expert_ids > kTileTable) return false;
   return (long long)a.num_tokens * a.topk >= 96LL * a.experts;
 }
 

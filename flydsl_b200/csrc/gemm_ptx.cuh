@@ -311,6 +311,65 @@ struct TileSched {
   }
 };
 
+// Block-wide exclusive scan over THREADS threads: running maximum (from -1) or running sum.
+template <bool MAX, int THREADS>
+__device__ __forceinline__ int block_scan_excl(int v, int* scratch, int* total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int inc = v;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const int o = __shfl_up_sync(0xffffffffu, inc, off);
+    if (lane >= off) inc = MAX ? max(inc, o) : inc + o;
+  }
+  if (lane == 31) scratch[warp] = inc;
+  __syncthreads();
+  int before = MAX ? -1 : 0, all = before;
+  for (int w = 0; w < THREADS / 32; ++w) {
+    if (w == warp) before = all;
+    all = MAX ? max(all, scratch[w]) : all + scratch[w];
+  }
+  const int prev = __shfl_up_sync(0xffffffffu, inc, 1);
+  *total = all;
+  if (lane == 0) return before;
+  return MAX ? max(before, prev) : before + prev;
+}
+// Row tiles of a launch: an expert's row blocks are contiguous in sorted order, and every `bpt`-th of them starts a
+// tile of up to bpt blocks.  table[tile] = first row block | (row blocks - 1) << 12.  Returns the number of tiles; the
+// caller synchronises the block before it reads the table.  scratch: two rows of 32 ints.
+constexpr int kTileTable = 4096;                 // row blocks the table covers
+template <int THREADS>
+__device__ __forceinline__ int build_tile_table(const GemmArgs& a, int valid_rows, int bpt, uint16_t* table,
+                                                int (*scratch)[32]) {
+  const int* ex = a.sorted_expert_ids;
+  const int nblk = min((valid_rows + a.tile_m - 1) / a.tile_m, kTileTable);
+  const int per = (nblk + THREADS - 1) / THREADS;
+  const int b0 = min(int(threadIdx.x) * per, nblk), b1 = min(b0 + per, nblk);
+  int run = -1;                                  // last start of an expert's run inside this thread's blocks
+  for (int b = b0; b < b1; ++b)
+    if (b == 0 || __ldg(ex + b) != __ldg(ex + b - 1)) run = b;
+  int unused, total;
+  const int run_before = block_scan_excl<true, THREADS>(run, scratch[0], &unused);
+  int starts = 0;
+  run = run_before;
+  for (int b = b0; b < b1; ++b) {
+    const int e = __ldg(ex + b);
+    if (b == 0 || e != __ldg(ex + b - 1)) run = b;
+    if (((b - run) & (bpt - 1)) == 0 && e >= 0 && e < a.experts) ++starts;
+  }
+  int at = block_scan_excl<false, THREADS>(starts, scratch[1], &total);
+  run = run_before;
+  for (int b = b0; b < b1; ++b) {
+    const int e = __ldg(ex + b);
+    if (b == 0 || e != __ldg(ex + b - 1)) run = b;
+    if (((b - run) & (bpt - 1)) == 0 && e >= 0 && e < a.experts) {
+      int nb = 1;
+      while (nb < bpt && b + nb < nblk && __ldg(ex + b + nb) == e) ++nb;
+      table[at++] = uint16_t(b | ((nb - 1) << 12));
+    }
+  }
+  return total;
+}
+
 // ------------------------------------------------------------------------------ host
 // Tensor maps of both operands: boxes of `a_box_rows` rows of A and of `b_box_rows` weight rows, 128 bytes of K wide.
 int make_gemm_maps(int stage, const GemmArgs& a, int a_box_rows, int b_box_rows, CUtensorMap* map_a, CUtensorMap* map_b);

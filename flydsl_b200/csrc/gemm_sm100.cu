@@ -86,7 +86,13 @@ struct __align__(16) SmemCtrl {
 template <int STAGE> constexpr size_t smem_bytes() {
   return size_t(RingDepth<STAGE>::value) * kStageBytes + Staging<STAGE>::bytes + sizeof(SmemCtrl) + 1024;
 }
-static_assert(smem_bytes<1>() <= 232448 && smem_bytes<2>() <= 232448, "shared memory budget of one SM exceeded");
+// Table of merged row tiles (MERGE instantiations), behind the control block.
+struct MergeTable {
+  int scan[2][32];
+  uint16_t table[kTileTable];
+};
+static_assert(smem_bytes<1>() + sizeof(MergeTable) <= 232448 && smem_bytes<2>() + sizeof(MergeTable) <= 232448,
+              "shared memory budget of one SM exceeded");
 
 // Optional whole-kernel wait accounting (build with -DFLYMOE_PROF, `python -m flydsl_b200.build
 // --prof`): every CTA's producer thread, MMA thread and first epilogue thread add up the cycles they
@@ -116,7 +122,9 @@ __device__ long long g_prof[256][3][8];
 // ROW_DST (stage 2 only): every output row goes to a caller-given address instead of out[t*k+s].  A
 // separate instantiation, so that the common kernel's register allocation is not touched.
 // GATHER: a separate instantiation, so that the kernels reading sorted rows keep their register allocation.
-template <int STAGE, bool ROW_DST, int SCALING, bool GATHER>
+// MERGE: consecutive row blocks of one expert (16, 32 or 64 rows each) run as one tile of up to 128 rows, so that the
+// expert's weights are fetched and multiplied once for all of them instead of once per block.
+template <int STAGE, bool ROW_DST, int SCALING, bool GATHER, bool MERGE>
 __global__ void __launch_bounds__(kNumThreads, 1)
 moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                       const GemmArgs a, const int group_m) {
@@ -136,8 +144,13 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   constexpr bool gather = GATHER;
   // Outputs that leave through the staging slots (everything except 16-bit stage-1 and fp32 stage-2 output)
   const bool uses_staging = STAGE == 1 ? a.out_dtype == FLYMOE_E4M3 : a.out_dtype != FLYMOE_F32;
+  MergeTable* merge = reinterpret_cast<MergeTable*>(ctrl + 1);
   TileSched sched;
-  sched.num_mblocks = (valid_rows + a.tile_m - 1) / a.tile_m;
+  sched.num_mblocks = MERGE ? build_tile_table<kNumThreads>(a, valid_rows, BM / a.tile_m, merge->table, merge->scan)
+                            : (valid_rows + a.tile_m - 1) / a.tile_m;
+  // row tile -> its first row block and its rows
+  auto tile_block = [&](int m) -> int { return MERGE ? int(merge->table[m] & 0xfff) : m; };
+  auto tile_rows = [&](int m) -> int { return MERGE ? (int(merge->table[m] >> 12) + 1) * a.tile_m : a.tile_m; };
   sched.num_ntiles = STAGE == 1 ? a.n_dim / 128 : (a.n_dim + BN - 1) / BN;
   sched.total = sched.num_mblocks * sched.num_ntiles;
   sched.group_m = group_m;
@@ -184,21 +197,22 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       // ---------------------------------------------------------------- TMA producer
       int stage = 0;
       uint32_t phase = 0;
-      const uint32_t tx_bytes = (gather ? 0u : uint32_t(a.tile_m) * BK) + kBTileBytes;
       bool ok = true;
       PROF_DECL
       int mb_next = 0, n_next = 0, e_next = -1;
       if (int(blockIdx.x) < sched.total) {
         sched.decode(blockIdx.x, mb_next, n_next);
-        e_next = __ldg(a.sorted_expert_ids + mb_next);
+        e_next = __ldg(a.sorted_expert_ids + tile_block(mb_next));
       }
       for (int t = blockIdx.x; t < sched.total && ok; t += gridDim.x) {
         const int mb = mb_next, n = n_next, e = e_next;
         if (t + int(gridDim.x) < sched.total) {          // next tile's expert id: loaded a whole tile early
           sched.decode(t + gridDim.x, mb_next, n_next);
-          e_next = __ldg(a.sorted_expert_ids + mb_next);
+          e_next = __ldg(a.sorted_expert_ids + tile_block(mb_next));
         }
         if (e < 0 || e >= a.experts) continue;
+        const int row0 = tile_block(mb) * a.tile_m, rows = tile_rows(mb);
+        const uint32_t tx_bytes = (gather ? 0u : uint32_t(rows) * BK) + kBTileBytes;
         for (int kb = 0; kb < KB; ++kb) {
           PROF_START
           if (!mbar_wait(smem_u32(&ctrl->empty[stage]), phase ^ 1, abort_flag, a.status, 1, 64)) { ok = false; break; }
@@ -207,7 +221,10 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           const uint32_t sa = smem_u32(smem + size_t(stage) * kStageBytes);
           const uint32_t sb = sa + kATileBytes;
           mbar_expect_tx(full, tx_bytes);
-          if (!gather) tma_load_2d(sa, &tmap_a, full, kb * BK, mb * a.tile_m);
+          if (!gather) tma_load_2d(sa, &tmap_a, full, kb * BK, row0);
+          if (MERGE && !gather)
+            for (int m = a.tile_m; m < rows; m += a.tile_m)
+              tma_load_2d(sa + uint32_t(m) * BK, &tmap_a, full, kb * BK, row0 + m);
           if (STAGE == 1) {
             tma_load_3d(sb, &tmap_b, full, kb * BK, n * 128, e);
             tma_load_3d(sb + 128 * BK, &tmap_b, full, kb * BK, a.n_dim + n * 128, e);
@@ -228,13 +245,13 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         int mb_next = 0, n_next = 0, e_next = -1;
         if (int(blockIdx.x) < sched.total) {
           sched.decode(blockIdx.x, mb_next, n_next);
-          e_next = __ldg(a.sorted_expert_ids + mb_next);
+          e_next = __ldg(a.sorted_expert_ids + tile_block(mb_next));
         }
         for (int t = blockIdx.x; t < sched.total; t += gridDim.x) {
           const int e = e_next;
           if (t + int(gridDim.x) < sched.total) {
             sched.decode(t + gridDim.x, mb_next, n_next);
-            e_next = __ldg(a.sorted_expert_ids + mb_next);
+            e_next = __ldg(a.sorted_expert_ids + tile_block(mb_next));
           }
           if (e < 0 || e >= a.experts) continue;
           for (int kb = 0; kb < KB; ++kb) {
@@ -281,7 +298,7 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       int mb_next = 0, n_next = 0, e_next = -1;
       if (int(blockIdx.x) < sched.total) {
         sched.decode(blockIdx.x, mb_next, n_next);
-        e_next = __ldg(a.sorted_expert_ids + mb_next);
+        e_next = __ldg(a.sorted_expert_ids + tile_block(mb_next));
       }
       constexpr uint32_t kSlotBytes = STAGE == 1 ? 64u : 256u;
       const bool bf = a.out_dtype == FLYMOE_BF16;
@@ -289,7 +306,7 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         const int e = e_next, n = n_next;
         if (t + int(gridDim.x) < sched.total) {
           sched.decode(t + gridDim.x, mb_next, n_next);
-          e_next = __ldg(a.sorted_expert_ids + mb_next);
+          e_next = __ldg(a.sorted_expert_ids + tile_block(mb_next));
         }
         if (e < 0 || e >= a.experts) continue;
         if (!mbar_wait(smem_u32(&ctrl->stg_full), it & 1, abort_flag, a.status, 6, 64)) { ok = false; break; }
@@ -340,15 +357,16 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       for (int t = blockIdx.x; t < sched.total && ok; t += gridDim.x) {
         int mb, n;
         sched.decode(t, mb, n);
-        const int e = __ldg(a.sorted_expert_ids + mb);
+        const int e = __ldg(a.sorted_expert_ids + tile_block(mb));
         if (e < 0 || e >= a.experts) continue;
+        const int row0 = tile_block(mb) * a.tile_m, rows = tile_rows(mb);
         const uint8_t* src[4];
         uint32_t nbytes[4];                      // 16 = copy, 0 = zero-fill (pad row)
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int row = j * 32 + lane;
-          const int r = mb * a.tile_m + row;
-          const int id = (row < a.tile_m && r < valid_rows) ? __ldg(a.sorted_ids + r) : pad_id;
+          const int r = row0 + row;
+          const int id = (row < rows && r < valid_rows) ? __ldg(a.sorted_ids + r) : pad_id;
           const int tok = id_token(id), slot = id_slot(id);
           const bool valid = tok < a.num_tokens && slot < a.topk;
           const long long srow = a.a_layout == FLYMOE_ROWS_BY_TOKEN ? (long long)tok
@@ -363,7 +381,7 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int row = j * 32 + lane;
-            if (row < a.tile_m) {
+            if (row < rows) {
               const uint8_t* g = src[j] + kb * BK;
               const uint32_t d = sa + uint32_t(row) * 128u;
 #pragma unroll
@@ -389,7 +407,6 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     const int wg = (warp - 4) >> 2;          // 0 or 1
     const int q = warp & 3;                  // TMEM lane quadrant of this warp
     const int row_in_tile = q * 32 + lane;
-    const bool warp_active = q * 32 < a.tile_m;
     const uint32_t lane_base = uint32_t(q * 32) << 16;
     int acc = 0;
     uint32_t acc_phase = 0;
@@ -405,9 +422,9 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
     int mb_next = 0, n_next = 0, e_next = -1, id_next = pad_id;
     auto load_routing = [&](int tt) {
       sched.decode(tt, mb_next, n_next);
-      e_next = __ldg(a.sorted_expert_ids + mb_next);
-      const int rr = mb_next * a.tile_m + row_in_tile;
-      id_next = (row_in_tile < a.tile_m && rr < valid_rows) ? __ldg(a.sorted_ids + rr) : pad_id;
+      e_next = __ldg(a.sorted_expert_ids + tile_block(mb_next));
+      const int rr = tile_block(mb_next) * a.tile_m + row_in_tile;
+      id_next = (row_in_tile < tile_rows(mb_next) && rr < valid_rows) ? __ldg(a.sorted_ids + rr) : pad_id;
     };
     if (int(blockIdx.x) < sched.total) load_routing(blockIdx.x);
     for (int t = blockIdx.x; t < sched.total && ok; t += gridDim.x) {
@@ -415,8 +432,10 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       if (t + int(gridDim.x) < sched.total) load_routing(t + gridDim.x);
       if (e < 0 || e >= a.experts) continue;
 
-      const int r = mb * a.tile_m + row_in_tile;
-      const bool in_tile = row_in_tile < a.tile_m && r < valid_rows;
+      const int rows = tile_rows(mb);
+      const bool warp_active = q * 32 < rows;
+      const int r = tile_block(mb) * a.tile_m + row_in_tile;
+      const bool in_tile = row_in_tile < rows && r < valid_rows;
       const int tok = id_token(id), slot = id_slot(id);
       const bool valid = in_tile && tok < a.num_tokens && slot < a.topk;
       long long sidx = 0;
@@ -793,23 +812,32 @@ int make_gemm_maps(int stage, const GemmArgs& a, int a_box_rows, int b_box_rows,
   return make_map(map_b, a.w, 3, bdims, bstrides, bbox);
 }
 
-template <int STAGE, bool ROW_DST, int SCALING, bool GATHER>
+template <int STAGE, bool ROW_DST, int SCALING, bool GATHER, bool MERGE>
 static int launch_kernel(int grid, cudaStream_t stream, const CUtensorMap& map_a, const CUtensorMap& map_b,
                          const GemmArgs& a, int group_m) {
-  auto* kernel = moe_gemm_sm100_kernel<STAGE, ROW_DST, SCALING, GATHER>;
-  FLYMOE_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         int(smem_bytes<STAGE>())));
-  kernel<<<grid, kNumThreads, smem_bytes<STAGE>(), stream>>>(map_a, map_b, a, group_m);
+  auto* kernel = moe_gemm_sm100_kernel<STAGE, ROW_DST, SCALING, GATHER, MERGE>;
+  constexpr size_t smem = smem_bytes<STAGE>() + (MERGE ? sizeof(MergeTable) : 0);
+  FLYMOE_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+  kernel<<<grid, kNumThreads, smem, stream>>>(map_a, map_b, a, group_m);
   FLYMOE_CUDA_CHECK(cudaGetLastError());
   return FLYMOE_OK;
 }
 
-template <int STAGE, bool ROW_DST, int SCALING>
+template <int STAGE, bool ROW_DST, int SCALING, bool MERGE>
 static int launch_one(int grid, cudaStream_t stream, const CUtensorMap& map_a, const CUtensorMap& map_b,
                       const GemmArgs& a, int group_m) {
   if (a.a_layout != FLYMOE_ROWS_SORTED)
-    return launch_kernel<STAGE, ROW_DST, SCALING, true>(grid, stream, map_a, map_b, a, group_m);
-  return launch_kernel<STAGE, ROW_DST, SCALING, false>(grid, stream, map_a, map_b, a, group_m);
+    return launch_kernel<STAGE, ROW_DST, SCALING, true, MERGE>(grid, stream, map_a, map_b, a, group_m);
+  return launch_kernel<STAGE, ROW_DST, SCALING, false, MERGE>(grid, stream, map_a, map_b, a, group_m);
+}
+
+// Row blocks of an expert are merged where it can have several: from a quarter of a block per expert on average (skewed
+// routing gives the busy ones many), up to the blocks the table covers.  128 tokens through 8 experts of 4096 x 14336,
+// top-2, 32-row blocks: 434 -> 327 us (8 tiles instead of about 12 per column); 777 tokens over 256 experts 2516 -> 2448.
+// Below a quarter there is next to nothing to merge (64 tokens over 256 experts: even), and the table costs a microsecond.
+static bool merge_blocks(const GemmArgs& a) {
+  return a.tile_m < BM && a.row_dst == nullptr && a.size_expert_ids <= kTileTable &&
+         4LL * a.num_tokens * a.topk >= (long long)a.tile_m * a.experts && a.experts > 1;
 }
 
 int choose_ksplit(int stage, const GemmArgs& a) {
@@ -841,7 +869,8 @@ int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {
                                 &map_a, &map_b);
   if (rc != FLYMOE_OK) return rc;
   const long long pairs = (long long)a.num_tokens * a.topk;
-  long long g = (pairs + (long long)a.experts * a.tile_m - 1) / ((long long)a.experts * a.tile_m);
+  const long long per_tile = (long long)a.experts * (merge_blocks(a) ? BM : a.tile_m);
+  long long g = (pairs + per_tile - 1) / per_tile;
   const int group_m = int(g < 1 ? 1 : (g > 16 ? 16 : g));
   const int split = a.ksplit > 0 ? a.ksplit : choose_ksplit(stage, a);
   if (split > 1) return launch_gemm_split(stage, a, map_a, map_b, group_m, split, stream);
@@ -849,12 +878,19 @@ int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {
   const long long max_tiles = (long long)a.size_expert_ids * ntiles;
   const int grid = int(max_tiles < ctas ? max_tiles : ctas);
   if (grid <= 0) return FLYMOE_OK;
+  if (merge_blocks(a)) {
+    if (per_token)
+      return stage == 1 ? launch_one<1, false, kScalePerToken, true>(grid, stream, map_a, map_b, a, group_m)
+                        : launch_one<2, false, kScalePerToken, true>(grid, stream, map_a, map_b, a, group_m);
+    return stage == 1 ? launch_one<1, false, kScaleBlock128, true>(grid, stream, map_a, map_b, a, group_m)
+                      : launch_one<2, false, kScaleBlock128, true>(grid, stream, map_a, map_b, a, group_m);
+  }
   if (per_token)
-    return stage == 1 ? launch_one<1, false, kScalePerToken>(grid, stream, map_a, map_b, a, group_m)
-                      : launch_one<2, false, kScalePerToken>(grid, stream, map_a, map_b, a, group_m);
-  if (stage == 1) return launch_one<1, false, kScaleBlock128>(grid, stream, map_a, map_b, a, group_m);
-  if (a.row_dst != nullptr) return launch_one<2, true, kScaleBlock128>(grid, stream, map_a, map_b, a, group_m);
-  return launch_one<2, false, kScaleBlock128>(grid, stream, map_a, map_b, a, group_m);
+    return stage == 1 ? launch_one<1, false, kScalePerToken, false>(grid, stream, map_a, map_b, a, group_m)
+                      : launch_one<2, false, kScalePerToken, false>(grid, stream, map_a, map_b, a, group_m);
+  if (stage == 1) return launch_one<1, false, kScaleBlock128, false>(grid, stream, map_a, map_b, a, group_m);
+  if (a.row_dst != nullptr) return launch_one<2, true, kScaleBlock128, false>(grid, stream, map_a, map_b, a, group_m);
+  return launch_one<2, false, kScaleBlock128, false>(grid, stream, map_a, map_b, a, group_m);
 }
 
 }  // namespace flymoe

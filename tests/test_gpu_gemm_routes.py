@@ -65,7 +65,7 @@ def _sort(ids, w, E, unit):
     return s, nblk
 
 
-@pytest.mark.parametrize("tile_m", [64, 128])
+@pytest.mark.parametrize("tile_m", [16, 32, 64, 128])
 @pytest.mark.parametrize("H,I,out", [(384, 256, "bf16"), (1024, 128, "f16")])
 def test_routed_blockscale_against_cuda_cores(H, I, out, tile_m):
     ids, tw = _routing(2)
@@ -103,7 +103,7 @@ def test_routed_blockscale_against_cuda_cores(H, I, out, tile_m):
     assert_close(c, rc, 1e-5, 1e-5 * float(rc.abs().max()), "stage 2 sums")
 
 
-@pytest.mark.parametrize("tile_m", [32, 128])
+@pytest.mark.parametrize("tile_m", [16, 32, 64, 128])
 @pytest.mark.parametrize("in_dtype", ["fp8", "int8"])
 def test_routed_pertoken_against_cuda_cores(in_dtype, tile_m):
     ids, tw = _routing(2)
