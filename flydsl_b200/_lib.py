@@ -28,6 +28,18 @@ DTYPE_CODE = {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16,
               torch.float8_e4m3fn: E4M3, torch.uint8: E4M3, torch.int8: I8}
 
 _P = c_void_p
+
+
+class LayerArgs(ctypes.Structure):
+    """flymoe_layer_args of include/flymoe.h, field by field."""
+    _fields_ = ([(n, _P) for n in ("logits", "xq", "x_scale", "w1", "w1_scale", "w2", "w2_scale", "topk_weights",
+                                   "topk_ids", "token_expert_ids", "sorted_ids", "sorted_weights", "sorted_expert_ids",
+                                   "num_valid_ids", "workspace", "xs", "a2", "a2_scale", "pair_out", "out")]
+                + [(n, c_int64) for n in ("workspace_elems", "sx_stride", "a2_scale_stride")]
+                + [(n, c_int32) for n in ("logits_dtype", "out_dtype", "tokens", "model_dim", "inter_dim", "experts",
+                                          "router_experts", "topk", "tile_m", "renormalize", "reduce", "impl")])
+
+
 _SIGNATURES = {
     "flymoe_abi_version": (c_int, []),
     "flymoe_error_string": (c_char_p, [c_int]),
@@ -53,6 +65,7 @@ _SIGNATURES = {
     "flymoe_moe_gemm2_pertoken": (c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P,
                                           c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                           c_int, c_int, c_int, c_int, c_int, _P]),
+    "flymoe_moe_layer": (c_int, [POINTER(LayerArgs), _P]),
     "flymoe_selftest_bounded_wait": (c_int, [c_int64, _P]),
     "flymoe_moe_gemm2_scatter_rows": (c_int, [_P, _P, _P, c_int64, _P, _P, _P, _P, _P, _P,
                                               c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,

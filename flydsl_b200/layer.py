@@ -211,11 +211,34 @@ class FusedMoEBlockscale:
             self.timing_events.append(("gemm2", t1, self._mark()))
 
     # ---------------------------------------------------------------- whole layer
+    def _forward_once(self, logits, xq, x_scale_t, tokens: int, out, stream: int) -> torch.Tensor:
+        """The checks of the pieces, then one call into the library for all of them."""
+        T, H, I = tokens, self.H, self.I
+        _lib.require_cuda("logits", logits, (torch.float32, torch.float16, torch.bfloat16), T * self.router_experts)
+        if T > self.max_tokens:
+            raise ValueError(f"tokens={T} exceeds max_tokens={self.max_tokens}")
+        _lib.require_cuda("xq", xq, _FP8, T * H)
+        _lib.require_cuda("x_scale_t", x_scale_t, (torch.float32,), (H // 128) * T)
+        out = self.out if out is None else out
+        _lib.require_cuda("out", out, (self.out_dtype,), T * H)
+        ptr = _lib.ptr
+        args = _lib.LayerArgs(
+            ptr(logits), ptr(xq), ptr(x_scale_t), ptr(self.w1q), ptr(self.w1_scale), ptr(self.w2q), ptr(self.w2_scale),
+            ptr(self.topk_weights), ptr(self.topk_ids), ptr(self.tei), ptr(self.sorted_ids), ptr(self.sorted_weights),
+            ptr(self.sorted_expert_ids), ptr(self.num_valid_ids), ptr(self.workspace), ptr(self.xs), ptr(self.a2q),
+            ptr(self.a2_scale), ptr(self.pair_out), ptr(out), self.workspace.numel(), x_scale_t.numel() // (H // 128),
+            self.cap_rows, _lib.DTYPE_CODE[logits.dtype], self.out_code, T, H, I, self.E, self.router_experts, self.topk,
+            self.tile_m, 1 if self.renormalize else 0, 1 if self.stage2_mode == "reduce" else 0, self.impl)
+        _lib.check(self.lib.flymoe_moe_layer(args, stream), "moe_layer")
+        return out[:T] if out.shape[0] != T else out
+
     def forward(self, logits: torch.Tensor, xq: torch.Tensor, x_scale_t: torch.Tensor,
                 out: torch.Tensor | None = None, stream=None) -> torch.Tensor:
         """logits [T, E] (f32/f16/bf16), xq e4m3 [T, H], x_scale_t f32 [H/128, T] -> out [T, H]."""
         tokens = logits.shape[0]
         h = _lib.stream_handle(stream)
+        if self.stage2_mode != "rows" and self.timing_events is None:
+            return self._forward_once(logits, xq, x_scale_t, tokens, out, h)
         self.gate(logits, tokens, h)
         res = self.experts_forward(self.topk_ids, self.topk_weights, xq, x_scale_t, tokens, h, out)
         return res[:tokens] if res.shape[0] != tokens else res

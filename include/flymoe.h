@@ -289,6 +289,24 @@ int flymoe_selftest_bounded_wait(int64_t limit_ns, void* stream);
  * kernels/moe_blockscale_2stage.py:1165-1183). */
 int flymoe_set_gemm_cta_limit(int max_ctas);
 
+/* One forward pass of a whole block-scaled layer: the calls above in order (gating, sort, row gather for row
+ * blocks of 64 or 128 rows, stage 1 with fused requantisation, stage 2, and for `reduce` the weighted top-k
+ * reduce), for hosts where crossing into the library once per kernel costs more than the kernels do.  All
+ * buffers are the caller's; `xs` is only used for tile_m > 32 and `pair_out` only for reduce. */
+typedef struct flymoe_layer_args {
+  const void* logits;                 /* [tokens, router_experts] of logits_dtype */
+  const void* xq;                     /* e4m3 [tokens, model_dim] */
+  const float* x_scale;               /* f32 [model_dim/128, sx_stride] */
+  const void* w1; const float* w1_scale; const void* w2; const float* w2_scale;
+  float* topk_weights; int32_t* topk_ids; int32_t* token_expert_ids;
+  int32_t* sorted_ids; float* sorted_weights; int32_t* sorted_expert_ids; int32_t* num_valid_ids;
+  int32_t* workspace; void* xs; void* a2; float* a2_scale; void* pair_out; void* out;
+  int64_t workspace_elems, sx_stride, a2_scale_stride;
+  int32_t logits_dtype, out_dtype, tokens, model_dim, inter_dim, experts, router_experts, topk, tile_m, renormalize,
+      reduce, impl;
+} flymoe_layer_args;
+int flymoe_moe_layer(const flymoe_layer_args* args, void* stream);
+
 /* Y[t,:] = sum_s w[t,s] * X[row(t,s),:] with fp32 accumulation; row(t,s) = t*k+s, or
  * row_index[t*k+s] when row_index is given (negative entries are skipped); optional u8
  * valid_mask [T,k] and optional f32 weights [T,k] (NULL = 1).
