@@ -445,7 +445,9 @@ int launch_gemm_pair(int stage, const GemmArgs& a, int ctas, cudaStream_t stream
   if (rc != FLYMOE_OK) return rc;
   // consecutive tiles (running at the same time) share one expert's weight tile
   const long long g = ((long long)a.num_tokens * a.topk + 2LL * BM * a.experts - 1) / (2LL * BM * a.experts);
-  const int group_m = int(g < 1 ? 1 : (g > 8 ? 8 : g));
+  // at least 2: an expert with a few rows beyond its first tile would otherwise stream its weights (more than L2 holds)
+  // once per tile.  1024 tokens, 8 experts of 4096 x 14336, top-2, bf16: 1143 -> 1078 us; 4 is no better than 2.
+  const int group_m = int(g < 2 ? 2 : (g > 8 ? 8 : g));
   const int ntiles = stage == 1 ? a.n_dim / 128 : ceil_div(a.n_dim, BN);
   const long long max_tiles = (long long)a.size_expert_ids * ntiles;
   int clusters = ctas / 2;
