@@ -246,7 +246,7 @@ class FusedMoEBlockscale:
     __call__ = forward
 
     def kernel_launches(self, tokens: int) -> int:
-        """Kernels this layer enqueues per forward (memset of the output not counted)."""
+        """Kernels this layer enqueues per forward."""
         sort = 1 if tokens * self.topk <= 8192 else 3
         return 1 + sort + (0 if self.gather_in_kernel else 1) + 1 + 1 + (1 if self.stage2_mode == "reduce" else 0)
 
