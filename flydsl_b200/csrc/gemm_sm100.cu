@@ -40,6 +40,9 @@
 // each row to a caller-given address, which may be in a peer GPU's memory.  The same
 // kernel with one expert and identity routing is the dense block-scaled GEMM.
 //
+// Two other kernels take what this one is not good at: gemm_split.cu launches with few tiles (a
+// cluster of CTAs shares K), gemm_pair.cu per-token scaling with many rows per expert (CTA pairs).
+//
 // Every wait is bounded: when one gives up it raises the CTA's abort flag and the
 // device status word, every role drains out, TMEM is released and the kernel returns.
 #include <cuda.h>
@@ -833,13 +836,17 @@ static int launch_one(int grid, cudaStream_t stream, const CUtensorMap& map_a, c
   return launch_kernel<STAGE, ROW_DST, SCALING, false, MERGE>(grid, stream, map_a, map_b, a, group_m);
 }
 
-// Row blocks of an expert are merged where it can have several: from a quarter of a block per expert on average (skewed
-// routing gives the busy ones many), up to the blocks the table covers.  128 tokens through 8 experts of 4096 x 14336,
-// top-2, 32-row blocks: 434 -> 327 us (8 tiles instead of about 12 per column); 777 tokens over 256 experts 2516 -> 2448.
-// Below a quarter there is next to nothing to merge (64 tokens over 256 experts: even), and the table costs a microsecond.
-static bool merge_blocks(const GemmArgs& a) {
-  return a.tile_m < BM && a.row_dst == nullptr && a.size_expert_ids <= kTileTable &&
-         4LL * a.num_tokens * a.topk >= (long long)a.tile_m * a.experts && a.experts > 1;
+// Row blocks of an expert are merged where that saves more than the table at kernel start costs (1-2 us): at a mean of
+// 0.8 blocks per expert about a quarter of the experts have a second one, and launches that stream 512 MB of weights or
+// more (80 us) gain from a quarter of a block on (a few per cent of the experts, or the busy ones of skewed routing).
+// 128 tokens through 8 experts of 4096 x 14336, top-2, 32-row blocks: 434 -> 327 us (8 tiles instead of about 12 per
+// column); 777 tokens over 256 experts 2516 -> 2448.  131 tokens over 64 experts of 2048 x 1024 (0.77 of a 16-row block,
+// 134 and 268 MB) lost 5 of 120 us to the table when it was merged.
+static bool merge_blocks(int stage, const GemmArgs& a) {
+  if (a.tile_m >= BM || a.row_dst != nullptr || a.size_expert_ids > kTileTable || a.experts < 2) return false;
+  const long long rows = (long long)a.num_tokens * a.topk, blocks = (long long)a.tile_m * a.experts;
+  const long long weight_bytes = (stage == 1 ? 2LL : 1LL) * a.n_dim * a.k_dim * a.experts;
+  return 5 * rows >= 4 * blocks || (weight_bytes >= (512LL << 20) && 4 * rows >= blocks);
 }
 
 int choose_ksplit(int stage, const GemmArgs& a) {
@@ -871,7 +878,7 @@ int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {
                                 &map_a, &map_b);
   if (rc != FLYMOE_OK) return rc;
   const long long pairs = (long long)a.num_tokens * a.topk;
-  const long long per_tile = (long long)a.experts * (merge_blocks(a) ? BM : a.tile_m);
+  const long long per_tile = (long long)a.experts * (merge_blocks(stage, a) ? BM : a.tile_m);
   long long g = (pairs + per_tile - 1) / per_tile;
   // at least 2: the second tile of an expert that has one more than the mean then runs beside the first
   const int group_m = int(g < 2 ? 2 : (g > 16 ? 16 : g));
@@ -881,7 +888,7 @@ int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {
   const long long max_tiles = (long long)a.size_expert_ids * ntiles;
   const int grid = int(max_tiles < ctas ? max_tiles : ctas);
   if (grid <= 0) return FLYMOE_OK;
-  if (merge_blocks(a)) {
+  if (merge_blocks(stage, a)) {
     if (per_token)
       return stage == 1 ? launch_one<1, false, kScalePerToken, true>(grid, stream, map_a, map_b, a, group_m)
                         : launch_one<2, false, kScalePerToken, true>(grid, stream, map_a, map_b, a, group_m);
