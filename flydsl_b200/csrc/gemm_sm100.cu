@@ -880,8 +880,7 @@ int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {
   const long long pairs = (long long)a.num_tokens * a.topk;
   const long long per_tile = (long long)a.experts * (merge_blocks(stage, a) ? BM : a.tile_m);
   long long g = (pairs + per_tile - 1) / per_tile;
-  // at least 2: the second tile of an expert that has one more than the mean then runs beside the first
-  const int group_m = int(g < 2 ? 2 : (g > 16 ? 16 : g));
+  const int group_m = int(g < 1 ? 1 : (g > 16 ? 16 : g));
   const int split = a.ksplit > 0 ? a.ksplit : choose_ksplit(stage, a);
   if (split > 1) return launch_gemm_split(stage, a, map_a, map_b, group_m, split, stream);
   const int ntiles = stage == 1 ? a.n_dim / 128 : ceil_div(a.n_dim, BN);
