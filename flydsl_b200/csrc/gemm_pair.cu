@@ -295,12 +295,12 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       const int col1 = wg * 32;                  // column of v1[0] within the first block, of v2[0] within the second
       {
         const bool i8 = a.in_dtype == FLYMOE_I8;
-        float sa = valid ? 1.f : 0.f;
-        if (valid && a.scale_a) {
+        float sa = 0.f;
+        if (valid) {
           const long long sidx = a.a_scale_layout == FLYMOE_ROWS_BY_TOKEN ? (long long)tok
                                : a.a_scale_layout == FLYMOE_ROWS_BY_PAIR ? (long long)tok * a.topk + slot
                                : a.a_scale_layout == FLYMOE_ROWS_BY_SLOT ? (long long)slot * a.num_tokens + tok : (long long)r;
-          sa = __ldg(a.scale_a + sidx);
+          sa = row_scale(a.scale_a, sidx);
         }
         const long long wrows = STAGE == 1 ? 2LL * a.n_dim : (long long)a.n_dim;
         const float* sw1 = a.scale_w + (long long)e * wrows + (STAGE == 1 ? n * 128 : n * BN) + col1;
@@ -308,11 +308,8 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
         const bool has2 = STAGE == 1 || n * BN + 128 < a.n_dim;
 #pragma unroll
         for (int j = 0; j < 32; j += 4) {
-          float4 s4 = make_float4(1.f, 1.f, 1.f, 1.f), u4 = s4;
-          if (a.scale_w) {
-            s4 = __ldg(reinterpret_cast<const float4*>(sw1 + j));
-            if (has2) u4 = __ldg(reinterpret_cast<const float4*>(sw2 + j));
-          }
+          const float4 s4 = col_scales4(a.scale_w, sw1 + j);
+          const float4 u4 = has2 ? col_scales4(a.scale_w, sw2 + j) : s4;
           const float c[4] = {s4.x, s4.y, s4.z, s4.w}, d[4] = {u4.x, u4.y, u4.z, u4.w};
 #pragma unroll
           for (int u = 0; u < 4; ++u) {

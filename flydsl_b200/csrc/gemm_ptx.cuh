@@ -133,6 +133,12 @@ __device__ __forceinline__ void gather_rows4(const GemmArgs& a, int first, int e
             : a.a_layout == FLYMOE_ROWS_BY_SLOT ? slot * a.num_tokens + tok : tok * a.topk + slot;
   }
 }
+// Per-token scaling, one rule for every kernel: a null table (16-bit operands; each of the two may be null by itself)
+// stands for ones.
+__device__ __forceinline__ float row_scale(const float* table, long long row) { return table ? __ldg(table + row) : 1.f; }
+__device__ __forceinline__ float4 col_scales4(const float* table, const float* at) {
+  return table ? __ldg(reinterpret_cast<const float4*>(at)) : make_float4(1.f, 1.f, 1.f, 1.f);
+}
 __device__ __forceinline__ void tcgen05_fence_before() {
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
 }

@@ -555,7 +555,7 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         acc ^= 1;
         if (work) {
           // 16-bit operands come without scales (null pointers): every factor is 1
-          const float sa = valid ? (a.scale_a ? __ldg(a.scale_a + sidx) : 1.f) : 0.f;
+          const float sa = valid ? row_scale(a.scale_a, sidx) : 0.f;
           const long long wrows = STAGE == 1 ? 2LL * a.n_dim : (long long)a.n_dim;
           // weight-row scales of this thread's two 64-column halves (the same addresses in every lane)
           const float* sw0 = a.scale_w + (long long)e * wrows + (STAGE == 1 ? n * 128 + wg * 64 : n * BN + wg * 128);
@@ -566,7 +566,7 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             const float* sw = h == 0 ? sw0 : sw1;
 #pragma unroll
             for (int j = 0; j < 64; j += 4) {
-              const float4 s4 = a.scale_w ? __ldg(reinterpret_cast<const float4*>(sw + j)) : make_float4(1.f, 1.f, 1.f, 1.f);
+              const float4 s4 = col_scales4(a.scale_w, sw + j);
               const float c[4] = {s4.x, s4.y, s4.z, s4.w};
 #pragma unroll
               for (int u = 0; u < 4; ++u) {

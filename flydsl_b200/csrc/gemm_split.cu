@@ -354,17 +354,15 @@ moe_gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 #pragma unroll
               for (int j = 0; j < 8; ++j) f[j] = __int2float_rn(isum[j]);
             }
-            const float sa = a.scale_a ? __ldg(a.scale_a + scale_row(r, id)) : 1.f;
-            if (a.scale_w) {
-              const long long wrows = STAGE == 1 ? 2LL * a.n_dim : (long long)a.n_dim;
-              const float* sw = a.scale_w + (long long)e * wrows + (STAGE == 1 ? n * 128 : n * BN) + lane * 4;
-              const bool second = STAGE == 1 || n * BN + 128 + lane * 4 < a.n_dim;
-              const float4 s0 = __ldg(reinterpret_cast<const float4*>(sw));
-              const float4 s1 = second ? __ldg(reinterpret_cast<const float4*>(sw + (STAGE == 1 ? a.n_dim : 128))) : s0;
-              const float c[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
+            const float sa = row_scale(a.scale_a, scale_row(r, id));
+            const long long wrows = STAGE == 1 ? 2LL * a.n_dim : (long long)a.n_dim;
+            const float* sw = a.scale_w + (long long)e * wrows + (STAGE == 1 ? n * 128 : n * BN) + lane * 4;
+            const bool second = STAGE == 1 || n * BN + 128 + lane * 4 < a.n_dim;
+            const float4 s0 = col_scales4(a.scale_w, sw);
+            const float4 s1 = second ? col_scales4(a.scale_w, sw + (STAGE == 1 ? a.n_dim : 128)) : s0;
+            const float c[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
-              for (int j = 0; j < 8; ++j) f[j] *= sa * c[j];
-            }
+            for (int j = 0; j < 8; ++j) f[j] *= sa * c[j];
           }
         }
         const float wgt = (a.doweight && valid) ? __ldg(a.sorted_weights + r) : 1.f;

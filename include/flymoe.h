@@ -170,8 +170,8 @@ int flymoe_moe_gemm2(void* out, const void* a2, const float* scale_a, int64_t sa
  * Replace kernels/moe_gemm_2stage.py:90-108 (compile_moe_gemm1, launcher :1730-1745) and
  * :1780-1796 (compile_moe_gemm2, launcher :3151-3166) for in_dtype "fp8", "int8", "int8smooth",
  * "fp16" and "bf16".  in_dtype E4M3, I8 (signed 8-bit operands, exact int32 accumulation), or
- * F16 / BF16 (16-bit operands and weights, tcgen05 kernel only; their scale pointers may be null,
- * which means every scale is 1, as in the reference where these variants carry no scales).
+ * F16 / BF16 (16-bit operands and weights, tcgen05 kernel only; their scale pointers may be null, each
+ * by itself, which means scales of 1, as in the reference where these variants carry no scales).
  * Stage 1: x [T,H] (x_layout BY_TOKEN), [k*T,H] slot-major (BY_SLOT: "int8smooth"), [T*k,H] (BY_PAIR)
  * or rows already in sorted order (SORTED); scale_x f32 [T] (x_scale_layout BY_TOKEN), [k*T] (BY_SLOT), [T*k] (BY_PAIR)
  * or per sorted row; w [E,2I,H] row-major, scale_w f32 [E*2I]; out F16/BF16 [T*k,I]
