@@ -45,6 +45,13 @@ struct GemmArgs {
   int* status;                 // device status word (bounded waits report here)
 };
 
+// CTA pairs share a tile of `blocks` row blocks: rows of it that CTA `rank` (0 or 1) loads and owns, at most 128.
+// Never more than the tile has, so nothing is read behind the last row block that the sort filled.
+__host__ __device__ constexpr int pair_rows(int blocks, int tile_m, int rank) {
+  const int rows = blocks * tile_m - rank * 128;
+  return rows < 0 ? 0 : (rows > 128 ? 128 : rows);
+}
+
 int launch_gemm_simt(int stage, const GemmArgs& args, cudaStream_t stream);
 int launch_gemm_sm100(int stage, const GemmArgs& args, cudaStream_t stream);
 // CTAs that launch_gemm_sm100 would give one tile (1: the one-CTA-per-tile kernels).

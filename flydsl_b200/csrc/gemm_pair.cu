@@ -5,8 +5,8 @@
 // the pair's leader issues M=256 N=256 MMAs that read both halves.  With one scale per row and column the MMAs
 // accumulate over the whole K range, so the tensor cores are the bound once the operands arrive: 48 KB per K block
 // are 768 cycles at the 64 bytes a cycle an SM takes from L2, 32 KB are the 512 the MMAs need.
-//   warp 0      TMA producer: this CTA's A box (128 rows x 128 B) and 128 weight rows x 128 B per K block.  The loads
-//               of both CTAs complete on the leader's full barrier.
+//   warp 0      TMA producer: this CTA's A rows (one or two boxes of a row block x 128 B) and 128 weight rows x 128 B
+//               per K block.  The loads of both CTAs complete on the leader's full barrier.
 //   warp 1      (leader) MMA issuer: four M=256 N=256 MMAs per K block into one of two TMEM stages.
 //   warp 2      store warp: one bulk store / bulk reduction per finished output row.
 //   warps 4-19  epilogue: four warpgroups; each thread owns one row and 2 x 32 of the tile's columns.
@@ -147,14 +147,15 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
   sched.total = sched.num_mblocks * sched.num_ntiles;
   sched.group_m = group_m;
   const int first_tile = int(blockIdx.x) >> 1, tile_step = int(gridDim.x) >> 1;
-  // tile -> N tile, expert, this CTA's first sorted row and how many rows it has (<= 0: none, at most 128 used)
-  auto tile_at = [&](int t, int& n, int& e, int& rows) -> int {
+  // tile -> N tile, expert, this CTA's first sorted row and how many rows it has
+  auto tile_at = [&](int t, int& n, int& e, int& rows, int* other_rows = nullptr) -> int {
     int p;
     sched.decode(t, p, n);
     const uint32_t entry = ctrl->table[p];
     const int b = int(entry & 0xfff);
     e = __ldg(a.sorted_expert_ids + b);
-    rows = (int(entry >> 12) + 1) * a.tile_m - rank * BM;
+    rows = pair_rows(int(entry >> 12) + 1, a.tile_m, rank);
+    if (other_rows) *other_rows = pair_rows(int(entry >> 12) + 1, a.tile_m, 1 - rank);
     return b * a.tile_m + rank * BM;
   };
 
@@ -169,13 +170,14 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
       uint32_t phase = 0;
       bool ok = true;
       for (int t = first_tile; t < sched.total && ok; t += tile_step) {
-        int n, e, rows;
-        const int row0 = tile_at(t, n, e, rows);
+        int n, e, rows, other_rows;
+        const int row0 = tile_at(t, n, e, rows, &other_rows);
         const int wrow = STAGE == 1 ? rank * a.n_dim + n * 128 : n * BN + rank * 128;
         // The leader announces the bytes of both CTAs on its barrier (an arrival from the other CTA that names its own
         // share needs release or relaxed semantics at cluster scope; the release alone took ~1500 cycles a K block).
         // The other CTA's bytes may land before the announcement: the phase still waits for the leader's arrival.
-        const uint32_t tx_bytes = uint32_t(kBTileBytes) + uint32_t(kATileBytes) * (rows > BM ? 2u : 1u);
+        // The activations come in boxes of one row block: a 128-row box would read up to 64 rows past the last block.
+        const uint32_t tx_bytes = uint32_t(kBTileBytes) + uint32_t(rows + other_rows) * BK;
         for (int kb = 0; kb < KB; ++kb) {
           ok = warp_wait(smem_u32(&ctrl->empty[stage]), phase ^ 1, abort_flag, a.status, 1, 32);
           if (!ok) break;
@@ -184,6 +186,7 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           if (elect_one()) {
             if (rank == 0) mbar_expect_tx(smem_u32(&ctrl->full[stage]), tx_bytes);
             if (rows > 0) tma_load_2d_pair(sa, &tmap_a, full, kb * BK, row0);
+            if (rows > a.tile_m) tma_load_2d_pair(sa + uint32_t(a.tile_m) * BK, &tmap_a, full, kb * BK, row0 + a.tile_m);
             tma_load_3d_pair(sa + kATileBytes, &tmap_b, full, kb * BK, wrow, e);
           }
           __syncwarp();
@@ -438,7 +441,7 @@ bool use_pair_kernel(const GemmArgs& a) {
 
 int launch_gemm_pair(int stage, const GemmArgs& a, int ctas, cudaStream_t stream) {
   CUtensorMap map_a, map_b;
-  const int rc = make_gemm_maps(stage, a, BM, 128, &map_a, &map_b);
+  const int rc = make_gemm_maps(stage, a, a.tile_m, 128, &map_a, &map_b);
   if (rc != FLYMOE_OK) return rc;
   // consecutive tiles (running at the same time) share one expert's weight tile
   const long long g = ((long long)a.num_tokens * a.topk + 2LL * BM * a.experts - 1) / (2LL * BM * a.experts);
