@@ -193,6 +193,12 @@ moe_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_co
           if (++stage == kRing) { stage = 0; phase ^= 1; }
         }
       }
+      // Nothing else waits for the last releases of the ring, which are the leader's MMAs arriving in BOTH CTAs: they have
+      // to land before this CTA's shared memory goes away.
+      for (int i = 0; i < kRing && ok; ++i) {
+        ok = warp_wait(smem_u32(&ctrl->empty[stage]), phase ^ 1, abort_flag, a.status, 1, 32);
+        if (++stage == kRing) { stage = 0; phase ^= 1; }
+      }
     } else if (warp == 1 && rank == 0) {
       // ---------------------------------------------------------------- MMA issuer
       auto issue = [&](auto kind_c, uint32_t dtype_bits) {
