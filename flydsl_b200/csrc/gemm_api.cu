@@ -1,6 +1,7 @@
 // C entry points of the two grouped-GEMM stages: argument validation and dispatch.
 #include "common.cuh"
 #include "gemm_args.cuh"
+#include "gemm_ptx.cuh"
 
 using namespace flymoe;
 
@@ -232,6 +233,19 @@ extern "C" int flymoe_moe_gemm2_scatter_rows(const uint64_t* row_dst, const void
                     sorted_ids, sorted_expert_ids, sorted_weights, num_valid_ids, num_tokens, model_dim, inter_dim,
                     size_expert_ids, experts, topk, tile_m, doweight, out_dtype, 0, a_layout, a_scale_layout,
                     FLYMOE_IMPL_TCGEN05, FLYMOE_SCALE_BLOCK128, FLYMOE_E4M3, stream);
+}
+
+extern "C" int flymoe_gemm_ksplit(int stage, int scaling, int num_tokens, int topk, int n_dim, int k_bytes,
+                                  int size_expert_ids, int tile_m, const int32_t* resident) {
+  GemmArgs a{};
+  a.scaling = scaling;
+  a.num_tokens = num_tokens;
+  a.topk = topk;
+  a.n_dim = n_dim;
+  a.k_dim = k_bytes;
+  a.size_expert_ids = size_expert_ids;
+  a.tile_m = tile_m;
+  return resident != nullptr ? plan_ksplit(stage, a, resident) : choose_ksplit(stage, a);
 }
 
 // ---------------------------------------------------------------------------------------------

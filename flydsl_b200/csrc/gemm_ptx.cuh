@@ -379,8 +379,12 @@ __device__ __forceinline__ int build_tile_table(const GemmArgs& a, int valid_row
 // ------------------------------------------------------------------------------ host
 // Tensor maps of both operands: boxes of `a_box_rows` rows of A and of `b_box_rows` weight rows, 128 bytes of K wide.
 int make_gemm_maps(int stage, const GemmArgs& a, int a_box_rows, int b_box_rows, CUtensorMap* map_a, CUtensorMap* map_b);
-// How many CTAs (one cluster) share a tile's K range; 1 = the one-CTA-per-tile kernel.
-int plan_ksplit(int stage, const GemmArgs& a, int ctas);
+// Cluster sizes 1, 2, 4, 8: how many CTAs share a tile's K range, given how many clusters of each size run at once
+// (0 = that size cannot run); 1 = the one-CTA-per-tile kernel.
+constexpr int kClusterSizes = 4;
+int plan_ksplit(int stage, const GemmArgs& a, const int* clusters);
+// Fills clusters[1..3] for the current device.
+void split_residency(int stage, int scaling, int* clusters);
 int launch_gemm_split(int stage, const GemmArgs& a, const CUtensorMap& map_a, const CUtensorMap& map_b, int group_m,
                       int split, cudaStream_t stream);
 bool use_pair_kernel(const GemmArgs& a);

@@ -852,7 +852,9 @@ static bool merge_blocks(int stage, const GemmArgs& a) {
 int choose_ksplit(int stage, const GemmArgs& a) {
   // a caller that leaves other kernels some SMs gets no clusters
   if (g_cta_limit > 0 && g_cta_limit < sm_count()) return 1;
-  return plan_ksplit(stage, a, sm_count());
+  int clusters[kClusterSizes] = {sm_count()};
+  split_residency(stage, a.scaling, clusters);
+  return plan_ksplit(stage, a, clusters);
 }
 
 int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {

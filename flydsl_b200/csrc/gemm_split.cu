@@ -436,35 +436,52 @@ moe_gemm_split_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
 
 // ------------------------------------------------------------------------------ host
 template <int STAGE, int SCALING>
-static int launch_split(const GemmArgs& a, const CUtensorMap& map_a, const CUtensorMap& map_b, int group_m, int split,
-                        cudaStream_t stream) {
-  auto* kernel = moe_gemm_split_kernel<STAGE, SCALING>;
-  FLYMOE_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSplitSmem)));
-  cudaLaunchAttribute attr;
-  attr.id = cudaLaunchAttributeClusterDimension;
-  attr.val.clusterDim.x = unsigned(split);
-  attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+static cudaLaunchConfig_t split_config(int split, cudaLaunchAttribute* attr) {
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = unsigned(split);
+  attr->val.clusterDim.y = attr->val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(kNumThreads);
   cfg.gridDim = dim3(unsigned(split));
   cfg.dynamicSmemBytes = kSplitSmem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
+  cfg.attrs = attr;
   cfg.numAttrs = 1;
-  // clusters that fit on the GPU at once (asked for once per device and cluster size)
-  static std::atomic<int> resident[64][9];
+  return cfg;
+}
+
+// Clusters of `split` CTAs that fit on the GPU at once (asked for once per device and cluster size); 0 where such a
+// cluster cannot be scheduled at all, as in a context limited to part of the GPU.
+template <int STAGE, int SCALING>
+static int resident_clusters(int split) {
+  static std::atomic<int> known[64][9];                    // answer + 1
   int dev = 0;
-  FLYMOE_CUDA_CHECK(cudaGetDevice(&dev));
-  int clusters = dev >= 0 && dev < 64 ? resident[dev][split].load(std::memory_order_relaxed) : 0;
-  if (clusters == 0) {
-    FLYMOE_CUDA_CHECK(cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg));
-    if (clusters < 1) clusters = 1;
-    if (dev >= 0 && dev < 64) resident[dev][split].store(clusters, std::memory_order_relaxed);
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  int n = known[dev][split].load(std::memory_order_relaxed) - 1;
+  if (n >= 0) return n;
+  auto* kernel = moe_gemm_split_kernel<STAGE, SCALING>;
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = split_config<STAGE, SCALING>(split, &attr);
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSplitSmem)) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
   }
+  known[dev][split].store(n + 1, std::memory_order_relaxed);
+  return n;
+}
+
+template <int STAGE, int SCALING>
+static int launch_split(const GemmArgs& a, const CUtensorMap& map_a, const CUtensorMap& map_b, int group_m, int split,
+                        cudaStream_t stream) {
+  auto* kernel = moe_gemm_split_kernel<STAGE, SCALING>;
+  FLYMOE_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSplitSmem)));
   const int ntiles = STAGE == 1 ? a.n_dim / 128 : ceil_div(a.n_dim, BN);
   const long long tiles = (long long)a.size_expert_ids * ntiles;
-  if (tiles < clusters) clusters = int(tiles);
-  cfg.gridDim = dim3(unsigned(clusters * split));
+  const int resident = resident_clusters<STAGE, SCALING>(split);     // at least one, or the plan would not say `split`
+  cudaLaunchAttribute attr;
+  cudaLaunchConfig_t cfg = split_config<STAGE, SCALING>(split, &attr);
+  cfg.gridDim = dim3(unsigned((tiles < resident ? int(tiles) : resident) * split));
+  cfg.stream = stream;
   FLYMOE_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, map_a, map_b, a, group_m, split));
   return FLYMOE_OK;
 }
@@ -478,7 +495,14 @@ int launch_gemm_split(int stage, const GemmArgs& a, const CUtensorMap& map_a, co
                     : launch_split<2, kScaleBlock128>(a, map_a, map_b, group_m, split, stream);
 }
 
-int plan_ksplit(int stage, const GemmArgs& a, int ctas) {
+void split_residency(int stage, int scaling, int* clusters) {
+  for (int i = 1, s = 2; i < kClusterSizes; ++i, s *= 2)
+    clusters[i] = scaling == FLYMOE_SCALE_PER_TOKEN
+                      ? (stage == 1 ? resident_clusters<1, kScalePerToken>(s) : resident_clusters<2, kScalePerToken>(s))
+                      : (stage == 1 ? resident_clusters<1, kScaleBlock128>(s) : resident_clusters<2, kScaleBlock128>(s));
+}
+
+int plan_ksplit(int stage, const GemmArgs& a, const int* clusters) {
   if (a.tile_m > kSplitMaxRows || a.row_dst != nullptr) return 1;
   const int KB = a.k_dim / BK;
   const long long pairs = (long long)a.num_tokens * a.topk;
@@ -490,9 +514,11 @@ int plan_ksplit(int stage, const GemmArgs& a, int ctas) {
   // stay with the kernel that has no exchange.
   int best = 1;
   double best_cost = 1e30;
-  for (int s = 1; s <= 8 && s <= KB; s *= 2) {
-    const long long slots = ctas / s;
-    if (slots < 1) break;
+  for (int i = 0, s = 1; i < kClusterSizes && s <= KB; ++i, s *= 2) {
+    // Clusters do not cross GPCs: 148 SMs ran 74 of 2, 33 of 4 and 15 of 8 at once.  Counting SMs / 8 = 18 instead, the
+    // 18 tiles of a dense M=64 N=4608 K=7168 were planned as one round of 8 and ran as two: 26.1 us, 18.4 as one of 4.
+    const long long slots = clusters[i];
+    if (slots < 1) continue;
     const double rounds = double((tiles + slots - 1) / slots);
     const double cost = rounds * (double((KB + s - 1) / s) + (s == 1 ? 3.0 : 5.0));
     if (cost < 0.9 * best_cost) { best = s; best_cost = cost; }

@@ -289,6 +289,13 @@ int flymoe_selftest_bounded_wait(int64_t limit_ns, void* stream);
  * kernels/moe_blockscale_2stage.py:1165-1183). */
 int flymoe_set_gemm_cta_limit(int max_ctas);
 
+/* How many CTAs (1, 2, 4 or 8) share the K range of a tile in a tcgen05 launch of these sizes without per-row
+ * destinations: stage 1 or 2, n_dim inter_dim (stage 1) or model_dim, k_bytes bytes of K per row (multiple of 128).
+ * resident: how many clusters of 1, 2, 4 and 8 CTAs run at once (0 = that size cannot run), or NULL for the current
+ * device.  A host-only query, for callers and tests that need to know which kernel a launch takes. */
+int flymoe_gemm_ksplit(int stage, int scaling, int num_tokens, int topk, int n_dim, int k_bytes,
+                       int size_expert_ids, int tile_m, const int32_t* resident);
+
 /* One forward pass of a whole block-scaled layer: the calls above in order (gating, sort, row gather for row
  * blocks of 64 or 128 rows, stage 1 with fused requantisation, stage 2, and for `reduce` the weighted top-k
  * reduce), for hosts where crossing into the library once per kernel costs more than the kernels do.  All

@@ -1,0 +1,33 @@
+"""Which cluster size shares the K range of a tile (host-only query; no GPU needed when the residency is given)."""
+import ctypes
+
+import pytest
+
+from flydsl_b200 import _lib
+
+B200 = (148, 74, 33, 15)                    # clusters of 1, 2, 4 and 8 CTAs that ran at once on one B200
+
+
+def ksplit(resident, tokens, n, k, *, topk=1, blocks=None, tile_m=64, stage=2):
+    blocks = (tokens + tile_m - 1) // tile_m if blocks is None else blocks
+    return _lib.load().flymoe_gemm_ksplit(stage, _lib.SCALE_BLOCK128, tokens, topk, n, k, blocks, tile_m,
+                                          ctypes.cast((ctypes.c_int32 * 4)(*resident), ctypes.c_void_p))
+
+
+def test_few_tiles_of_long_k_are_shared():
+    assert ksplit(B200, 64, 2112, 7168) == 8                            # 9 tiles of 56 K blocks
+    assert ksplit(B200, 64, 2112, 128) == 1                             # one K block: nothing to share
+    assert ksplit(B200, 64, 2112, 7168, tile_m=128) == 1                # 128-row blocks run on one CTA
+    assert ksplit(B200, 64 * 148, 2112, 7168) == 1                      # the tiles fill the GPU
+
+
+@pytest.mark.parametrize("size", [8, 4, 2])
+def test_a_size_that_cannot_run_is_not_chosen(size):
+    resident = [n if (1 << i) < size else 0 for i, n in enumerate(B200)]
+    assert ksplit(resident, 64, 2112, 7168) == size // 2
+
+
+def test_the_plan_counts_the_clusters_that_run_at_once():
+    # 18 tiles of 56 K blocks: one round of 18 clusters of 8, or two where only 15 run at once -- then one round of 4
+    assert ksplit((148, 74, 37, 18), 64, 4608, 7168) == 8
+    assert ksplit(B200, 64, 4608, 7168) == 4
