@@ -1,5 +1,6 @@
-"""Edges of the GEMM kernels' routes, through the launchers: the K range of a tile shared by a cluster (few tiles:
-row blocks of 16-64) and experts with many rows (row blocks of 64 and 128).
+"""Edges of the GEMM kernels' routes, through the launchers: dense shapes on the cluster (row blocks of 16-64, few
+tiles) and one-CTA kernels, and routed ones with enough rows per expert for merged row blocks and, with per-token scales
+and row blocks of 64 and 128, for CTA pairs.  Routed launches on the cluster kernel: test_gpu_gemm_split.py.
 
 References: the CPU oracle for dense shapes (16-bit results: one rounding step, 2^-8 / 2^-11 relative, plus fp32 sums
 in another order), and the CUDA-core implementation for routed ones."""
@@ -21,7 +22,7 @@ EPS = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11}
 
 
 # K = 128 (nothing to split), 256, 1152 (9 K blocks: uneven shares), 7168; N = 64 mod 128, 128 mod 256, whole tiles;
-# M around the row blocks, and around one and two 128-row blocks (pair with and without its second block)
+# M around the row blocks, and around one and two 128-row blocks (which never share K)
 @pytest.mark.parametrize("N,K", [(192, 128), (64, 256), (384, 1152), (2112, 7168)])
 @pytest.mark.parametrize("M,tile_m", [(1, 16), (16, 16), (17, 32), (64, 64), (96, 128), (128, 128), (129, 128),
                                       (257, 128), (640, 128)])
