@@ -303,6 +303,8 @@ extern "C" int64_t flymoe_moe_sorting_workspace_elems(int num_tokens, int num_ex
   bool one_block;
   flymoe::sort_plan(int(pairs), &seg_len, &nseg, &one_block);
   if (one_block) return 0;
+  // The kernels keep totals per block of eight segments and touch an eighth of this; the size stays one row per segment,
+  // which callers may have laid out, and with it what the allocation-free variant refuses.
   return int64_t(nseg) * num_experts + num_experts;
 }
 
