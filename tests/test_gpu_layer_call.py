@@ -43,3 +43,35 @@ def test_one_call_refuses_what_the_pieces_refuse():
         layer(logits, xq[:4], xs_t)
     with pytest.raises(ValueError, match="contiguous"):
         layer(logits, xq, xs_t.t())
+
+
+def _layer_and_inputs(cls):
+    cfg = wl.MoEConfig("call", 40, 256, 128, 6, 2, 11)
+    layer = cls(*wl.make_weights(cfg, device="cuda"), cfg.topk, max_tokens=cfg.tokens, tile_m=16, stage2_mode="reduce")
+    xq, xs_t = quant_act_1x128(wl.make_activations(cfg, device="cuda")[0])
+    return layer, wl.make_logits(cfg, device="cuda"), xq, xs_t
+
+
+class _FirstExperts(FusedMoEBlockscale):
+    """A router of its own: experts 0 and 1, equal weights."""
+
+    def gate(self, logits, tokens, stream):
+        self.topk_ids[:tokens] = torch.arange(self.topk, dtype=torch.int32, device=self.device)
+        self.topk_weights[:tokens] = 1.0 / self.topk
+
+
+def test_an_overridden_piece_is_used():
+    layer, logits, xq, xs_t = _layer_and_inputs(_FirstExperts)
+    got = layer(logits, xq, xs_t).clone()
+    T = logits.shape[0]
+    ids = torch.arange(2, dtype=torch.int32, device="cuda").repeat(T, 1)
+    tw = torch.full((T, 2), 0.5, device="cuda")
+    want = layer.experts_forward(ids, tw, xq, xs_t, T, torch.cuda.current_stream().cuda_stream)[:T]
+    assert torch.equal(got, want)
+    # a piece replaced on the object
+    plain, *_ = _layer_and_inputs(FusedMoEBlockscale)
+    calls = []
+    plain.experts_forward = lambda *a, **k: (calls.append(1), FusedMoEBlockscale.experts_forward(plain, *a, **k))[1]
+    plain(logits, xq, xs_t)
+    torch.cuda.synchronize()
+    assert calls == [1] and _lib.device_status() == 0
