@@ -169,6 +169,14 @@ def parity_check(cfg: wl.MoEConfig, tokens, logits_c, xq_c, xs_c, out_rows, fetc
             "ref_max_abs": round(float(ref.abs().max()), 4), "rtol": 2e-2, "atol": 2e-2, "ok": ok}
 
 
+def shared_k_note(lib, cfg, tile_m: int, stage: int, resident=None) -> str | None:
+    """Why a stage of the fused layer has no wait accounting: its launch takes the kernel that shares K in a cluster."""
+    n, k = (cfg.inter_dim, cfg.model_dim) if stage == 1 else (cfg.model_dim, cfg.inter_dim)
+    rows = cfg.tokens * cfg.topk + cfg.experts * tile_m - cfg.topk
+    ctas = lib.flymoe_gemm_ksplit(stage, 0, cfg.tokens, cfg.topk, n, k, (rows + tile_m - 1) // tile_m, tile_m, resident)
+    return None if ctas == 1 else f"clusters of {ctas} CTAs share K (moe_gemm_split_kernel), which keeps no wait accounting"
+
+
 def wait_accounting(args, cfg) -> None:
     """Mean cycles per 128-wide K block that each role of the grouped-GEMM kernels spends waiting, read
     from a library built with -DFLYMOE_PROF (FLYMOE_LIB=flydsl_b200/libflymoe_sm100_prof.so)."""
@@ -193,7 +201,11 @@ def wait_accounting(args, cfg) -> None:
     torch.cuda.synchronize()
     buf = np.zeros((256, 3, 8), dtype=np.int64)
 
-    def show(tag):
+    def show(stage, tag):
+        note = shared_k_note(lib, cfg, layer.tile_m, stage)
+        if note is not None:                       # the counters hold an earlier launch, or nothing
+            print(json.dumps({"kernel": tag, "workload": cfg.name, "unavailable": note}), flush=True)
+            return
         lib.flymoe_prof_read(buf.ctypes.data)
         b = buf[:torch.cuda.get_device_properties(dev).multi_processor_count].astype(np.float64)
         p, m, e = b[:, 0], b[:, 1], b[:, 2]
@@ -208,7 +220,7 @@ def wait_accounting(args, cfg) -> None:
                           "mma_issue_and_commit": round(m[:, 4].mean() / nkb, 1),
                           "epilogue_wait_mma": round(e[:, 1].mean() / nkb, 1),
                           "tile_end_cycles_per_tile": round(e[:, 2].mean() / max(e[:, 5].mean(), 1.0), 1)}), flush=True)
-    show("stage 2 (last launch of the layer)")
+    show(2, "stage 2 (last launch of the layer)")
     # stage 1 alone, so that its counters are the last ones written
     U = layer.tile_m
     cap = T * k + E * U - k
@@ -223,7 +235,7 @@ def wait_accounting(args, cfg) -> None:
             _lib.ROWS_BY_TOKEN if layer.gather_in_kernel else _lib.ROWS_SORTED, _lib.ROWS_BY_TOKEN, _lib.ROWS_SORTED,
             0, st), "moe_gemm1")
     torch.cuda.synchronize()
-    show("stage 1")
+    show(1, "stage 1")
 
 
 # ------------------------------------------------------------------------------------ GPU arm

@@ -31,3 +31,14 @@ def test_the_plan_counts_the_clusters_that_run_at_once():
     # 18 tiles of 56 K blocks: one round of 18 clusters of 8, or two where only 15 run at once -- then one round of 4
     assert ksplit((148, 74, 37, 18), 64, 4608, 7168) == 8
     assert ksplit(B200, 64, 4608, 7168) == 4
+
+
+def test_wait_accounting_is_not_read_for_the_cluster_kernel():
+    import bench
+    from flydsl_b200 import workloads as wl
+    lib, res = _lib.load(), ctypes.cast((ctypes.c_int32 * 4)(*B200), ctypes.c_void_p)
+    one_token = wl.MoEConfig("few tiles", 1, 4096, 14336, 8, 2, 0)
+    prefill = wl.MoEConfig("many tiles", 4096, 7168, 2048, 256, 8, 0)
+    assert "moe_gemm_split_kernel" in bench.shared_k_note(lib, one_token, 16, 2, res)
+    assert bench.shared_k_note(lib, one_token, 16, 1, res) is None            # 224 tiles fill the GPU
+    assert [bench.shared_k_note(lib, prefill, 128, s, res) for s in (1, 2)] == [None, None]
