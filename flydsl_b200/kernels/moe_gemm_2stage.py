@@ -36,7 +36,8 @@ runs.
 ``k_batch > 1`` (stage 1): the reference's split-K launches add the scaled gate and up sums, without
 activation and routing weight, to a caller-zeroed fp32 ``[tokens*topk, 2*inter]`` buffer and the caller
 finishes ``silu(gate)*up`` (:121-122; its test :582-587, :708-713).  The launcher built here keeps that
-output contract; K is not actually split (one CTA sums the whole K range and adds once per element).
+output contract; ``k_batch`` itself splits nothing: a launch sums the whole K range of a tile, in one CTA or in a cluster of
+them whose partial sums meet first, and adds once per element.
 
 Not built here: ``k_batch > 1`` with bf16 activations (bf16 partial sums) and group-wise scales with int8
 activations (``in_dtype="int4"`` with ``group_size > 0``) raise ``ValueError`` at build time; ``group_size`` other than 32 is rejected as in
@@ -85,7 +86,7 @@ def _check(in_dtype, group_size, k_batch, tile_m, tile_k, model_dim, inter_dim, 
         raise ValueError(f"k_batch must be >= 1, got {k_batch}")
     if k_batch > 1:
         # split-K launches keep the reference's OUTPUT contract (raw fp32 gate|up sums added to a zeroed
-        # [tokens*topk, 2*inter] buffer); K itself is not split here, one CTA owns the whole K range of a tile
+        # [tokens*topk, 2*inter] buffer); k_batch itself splits nothing: every element receives one addition
         if in_dtype in ("bf16", "int4_bf16"):
             raise ValueError("k_batch > 1 with bf16 activations accumulates bf16 partial sums in the reference; "
                              "that output format is not built here")

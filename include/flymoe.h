@@ -267,8 +267,8 @@ int flymoe_ep_plan_direct(const int64_t* counts, const int64_t* peer_base, int64
  * a e4m3 [M,K]; scale_a f32 [K/128, sa_stride] (the reference's transposed layout,
  * sa_stride >= M); b e4m3 [N,K] row-major; scale_b f32 [ceil(N/128), K/128]; c [M,N] of
  * out_dtype (F16/BF16).  K must be a multiple of 128, N a multiple of 64.
- * workspace: flymoe_blockscale_gemm_workspace_elems(M, tile_m) int32, rewritten by every
- * call (the routing arrays of the grouped kernel); tile_m 16/32/64/128. */
+ * workspace: flymoe_blockscale_gemm_workspace_elems(M, tile_m) int32, which any call may rewrite (the
+ * routing arrays of the grouped kernel; not needed where K is shared in a cluster); tile_m 16/32/64/128. */
 int64_t flymoe_blockscale_gemm_workspace_elems(int m, int tile_m);
 int flymoe_blockscale_gemm(void* c, const void* a, const float* scale_a, int64_t sa_stride,
                            const void* b, const float* scale_b, int32_t* workspace,
@@ -285,8 +285,8 @@ int flymoe_selftest_bounded_wait(int64_t limit_ns, void* stream);
 
 /* Caps the persistent grid of the two GEMM stages at max_ctas CTAs (0 restores one CTA per SM).
  * Process-wide.  For callers that run communication kernels next to the GEMMs (the
- * expert-parallel layer); the reference has no counterpart (its grid is one CTA per tile,
- * kernels/moe_blockscale_2stage.py:1165-1183). */
+ * expert-parallel layer): below the GPU's SM count it also keeps K from being shared in clusters.  The
+ * reference has no counterpart (its grid is one CTA per tile, kernels/moe_blockscale_2stage.py:1165-1183). */
 int flymoe_set_gemm_cta_limit(int max_ctas);
 
 /* How many CTAs (1, 2, 4 or 8) share the K range of a tile in a tcgen05 launch of these sizes without per-row
