@@ -66,6 +66,7 @@ _SIGNATURES = {
                                           c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int,
                                           c_int, c_int, c_int, c_int, c_int, _P]),
     "flymoe_gemm_ksplit": (c_int, [c_int, c_int, c_int, c_int, c_int, c_int, c_int, c_int, _P]),
+    "flymoe_gemm_merges_blocks": (c_int, [c_int] * 10),
     "flymoe_moe_layer": (c_int, [POINTER(LayerArgs), _P]),
     "flymoe_selftest_bounded_wait": (c_int, [c_int64, _P]),
     "flymoe_moe_gemm2_scatter_rows": (c_int, [_P, _P, _P, c_int64, _P, _P, _P, _P, _P, _P,

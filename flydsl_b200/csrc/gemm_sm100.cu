@@ -47,6 +47,7 @@
 // device status word, every role drains out, TMEM is released and the kernel returns.
 #include <cuda.h>
 #include <cudaTypedefs.h>
+#include <math.h>
 #include <stdio.h>
 #include <type_traits>
 
@@ -342,9 +343,12 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       // A K block's copies are completed two K blocks later (cp.async.wait_group), made visible to the
       // tensor cores' proxy (fence.proxy.async) and then signalled on the stage's full barrier, next to
       // the TMA thread's arrival for the weights.  Pad rows are zero-filled (source size 0).
-      // One warp issues every request, which keeps up with row blocks of 16 or 32 rows (decode); for
-      // 64 and 128 rows it is slower than gathering ahead of the launch (measured: stage 1 of the
-      // T=4096 layer 2.5 ms against 1.9 + 0.08 ms), so the host wrappers gather ahead for those.
+      // One warp issues every request, which keeps up with row blocks of 16 or 32 rows (decode); with
+      // 64 and 128 rows a K block takes longer here than in the tensor cores, so the host wrappers gather
+      // such blocks ahead of the launch (stage 1 of the T=4096 layer 2.5 ms against 1.9 + 0.08 ms).  Merged
+      // blocks of 16 or 32 rows still come through here, up to 1024 requests per K block: slower per tile
+      // (merge_blocks counts it), but instead of the weights once per block (333 tokens over 256 experts of
+      // 7168 x 2048, 16-row blocks, Zipf: 1332 us one by one, 500 merged).
       constexpr int kInFlight = 2;
       int stage = 0, pending = 0;
       uint32_t phase = 0;
@@ -836,17 +840,58 @@ static int launch_one(int grid, cudaStream_t stream, const CUtensorMap& map_a, c
   return launch_kernel<STAGE, ROW_DST, SCALING, false, MERGE>(grid, stream, map_a, map_b, a, group_m);
 }
 
-// Row blocks of an expert are merged where that saves more than the table at kernel start costs (1-2 us): at a mean of
-// 0.8 blocks per expert about a quarter of the experts have a second one, and launches that stream 512 MB of weights or
-// more (80 us) gain from a quarter of a block on (a few per cent of the experts, or the busy ones of skewed routing).
-// 128 tokens through 8 experts of 4096 x 14336, top-2, 32-row blocks: 434 -> 327 us (8 tiles instead of about 12 per
-// column); 777 tokens over 256 experts 2516 -> 2448.  131 tokens over 64 experts of 2048 x 1024 (0.77 of a 16-row block,
-// 134 and 268 MB) lost 5 of 120 us to the table when it was merged.
-static bool merge_blocks(int stage, const GemmArgs& a) {
+// Expected row tiles of an expert that receives `mean` rows on average, spread as under even routing (Poisson, tails by
+// the normal distribution).
+static double row_tiles(double mean, int unit) {
+  if (mean >= 4.0 * unit) return mean / unit + 0.5;
+  double n = 1.0 - exp(-mean);
+  for (int j = 1; j <= 8; ++j) {
+    const double p = 0.5 * erfc((j * unit + 0.5 - mean) / sqrt(2.0 * mean));
+    if (p < 1e-3) break;
+    n += p;
+  }
+  return n;
+}
+
+// Microseconds of a launch whose row tiles hold `rows` rows: rounds of tiles times (fill, tile end and K blocks).  One
+// warp fetches rows by index, so a gathered K block costs with its rows what 16 bytes per request cost.  Fitted to layers
+// of 8 experts of 1024 x 512 (1 and 2 rounds of 4 to 8 K blocks) and of 16 of 4096 x 1536 (2 to 50 rounds of 12 to 32).
+static double tile_rounds_us(double tiles, double rows, bool gather, int KB, int ctas) {
+  const double kblock = gather ? 0.6 + 0.008 * (rows - 16.0) : 0.6 + 0.0012 * rows;
+  return ceil(tiles / ctas) * (1.5 + 0.0375 * rows + KB * kblock);
+}
+
+// Row blocks of an expert are merged where fewer rounds of longer tiles are expected to take less time than the blocks
+// one by one, the table at kernel start (1.5 us) included.  Layers on one B200, whole calls in a CUDA graph, us one by
+// one -> merged, even routing:
+//   8 experts of 1024 x 512, top-2, 16-row blocks: 192 tokens 31 -> 39, 512 tokens 43 -> 51 (both left alone: the blocks
+//   fit one or two rounds, the merged tiles are one long one), 1024 tokens 69 -> 57, 2048 tokens 117 -> 66;
+//   16 experts of 4096 x 1536, top-2, 32-row blocks: 205 tokens 92 -> 100 (left alone), 384 tokens 123 -> 108, 2048 398 -> 235;
+//   64 experts of 2048 x 1024, top-6, 32-row blocks: 273 tokens 115 -> 123 (left alone), 341 tokens 143 -> 130;
+//   8 experts of 4096 x 14336, top-2, 128 tokens, 32-row blocks: 421 -> 302.
+// From 0.8 of a block per expert on, a launch that this expects to lose less than 3 % is merged all the same: skewed
+// routing has the busy experts' second blocks there already (205 tokens through that layer in 64-row blocks, Zipf:
+// 405 -> 303 merged; even 321 -> 323).
+// Launches that stream 512 MB of weights or more are merged from a quarter of a block per expert on.  Under even routing
+// no expert has a second block there, and the merging kernel is even to 6 % slower (42 to 102 tokens through the
+// 4096 x 14336 layer: 281 -> 292, 290 -> 301 us); under skewed routing the busy experts have many (the same 102 tokens,
+// Zipf, its first stage merged: 390 -> 323; 128 tokens over 256 experts of 7168 x 2048, 16-row blocks: 691 -> 315).
+static bool merge_blocks(int stage, const GemmArgs& a, int ctas) {
   if (a.tile_m >= BM || a.row_dst != nullptr || a.size_expert_ids > kTileTable || a.experts < 2) return false;
-  const long long rows = (long long)a.num_tokens * a.topk, blocks = (long long)a.tile_m * a.experts;
+  const long long rows = (long long)a.num_tokens * a.topk;
   const long long weight_bytes = (stage == 1 ? 2LL : 1LL) * a.n_dim * a.k_dim * a.experts;
-  return 5 * rows >= 4 * blocks || (weight_bytes >= (512LL << 20) && 4 * rows >= blocks);
+  if (weight_bytes >= (512LL << 20) && 4 * rows >= (long long)a.tile_m * a.experts) return true;
+  const double mean = double(rows) / a.experts;
+  const int ntiles = stage == 1 ? a.n_dim / 128 : ceil_div(a.n_dim, BN);
+  const double blocks = row_tiles(mean, a.tile_m), tiles = row_tiles(mean, BM);
+  const bool gather = a.a_layout != FLYMOE_ROWS_SORTED;
+  const double apart = tile_rounds_us(blocks * a.experts * ntiles, a.tile_m, gather, a.k_dim / BK, ctas);
+  // a tile holds its share of the blocks on average; a launch of one round takes as long as its longest tile
+  double tile_rows = a.tile_m * blocks / tiles;
+  if (tiles * a.experts * ntiles <= ctas) tile_rows = ceil((mean + sqrt(mean)) / a.tile_m) * a.tile_m;
+  if (tile_rows > BM) tile_rows = BM;
+  const double merged = tile_rounds_us(tiles * a.experts * ntiles, tile_rows, gather, a.k_dim / BK, ctas) + 1.5;
+  return merged < (mean >= 0.8 * a.tile_m ? 1.03 : 1.0) * apart;
 }
 
 int choose_ksplit(int stage, const GemmArgs& a) {
@@ -880,16 +925,17 @@ int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {
                                 &map_a, &map_b);
   if (rc != FLYMOE_OK) return rc;
   const long long pairs = (long long)a.num_tokens * a.topk;
-  const long long per_tile = (long long)a.experts * (merge_blocks(stage, a) ? BM : a.tile_m);
+  const int split = a.ksplit > 0 ? a.ksplit : choose_ksplit(stage, a);
+  const bool merge = split == 1 && merge_blocks(stage, a, ctas);
+  const long long per_tile = (long long)a.experts * (merge ? BM : a.tile_m);
   long long g = (pairs + per_tile - 1) / per_tile;
   const int group_m = int(g < 1 ? 1 : (g > 16 ? 16 : g));
-  const int split = a.ksplit > 0 ? a.ksplit : choose_ksplit(stage, a);
   if (split > 1) return launch_gemm_split(stage, a, map_a, map_b, group_m, split, stream);
   const int ntiles = stage == 1 ? a.n_dim / 128 : ceil_div(a.n_dim, BN);
   const long long max_tiles = (long long)a.size_expert_ids * ntiles;
   const int grid = int(max_tiles < ctas ? max_tiles : ctas);
   if (grid <= 0) return FLYMOE_OK;
-  if (merge_blocks(stage, a)) {
+  if (merge) {
     if (per_token)
       return stage == 1 ? launch_one<1, false, kScalePerToken, true>(grid, stream, map_a, map_b, a, group_m)
                         : launch_one<2, false, kScalePerToken, true>(grid, stream, map_a, map_b, a, group_m);
@@ -905,3 +951,17 @@ int launch_gemm_sm100(int stage, const GemmArgs& a, cudaStream_t stream) {
 }
 
 }  // namespace flymoe
+
+extern "C" int flymoe_gemm_merges_blocks(int stage, int num_tokens, int topk, int experts, int n_dim, int k_bytes,
+                                         int size_expert_ids, int tile_m, int x_layout, int ctas) {
+  flymoe::GemmArgs a{};
+  a.num_tokens = num_tokens;
+  a.topk = topk;
+  a.experts = experts;
+  a.n_dim = n_dim;
+  a.k_dim = k_bytes;
+  a.size_expert_ids = size_expert_ids;
+  a.tile_m = tile_m;
+  a.a_layout = x_layout;
+  return flymoe::merge_blocks(stage, a, ctas > 0 ? ctas : flymoe::sm_count()) ? 1 : 0;
+}

@@ -296,6 +296,12 @@ int flymoe_set_gemm_cta_limit(int max_ctas);
 int flymoe_gemm_ksplit(int stage, int scaling, int num_tokens, int topk, int n_dim, int k_bytes,
                        int size_expert_ids, int tile_m, const int32_t* resident);
 
+/* Whether a tcgen05 launch of these sizes that does not share K, has no per-row destinations and does not run on CTA
+ * pairs merges consecutive row blocks of an expert into tiles of up to 128 rows (1) or runs them one by one (0).
+ * x_layout: FLYMOE_ROWS_* of the launch's activations; ctas: CTAs of the launch, 0 = one per SM.  Host-only, as above. */
+int flymoe_gemm_merges_blocks(int stage, int num_tokens, int topk, int experts, int n_dim, int k_bytes,
+                              int size_expert_ids, int tile_m, int x_layout, int ctas);
+
 /* One forward pass of a whole block-scaled layer: the calls above in order (gating, sort, row gather for row
  * blocks of 64 or 128 rows, stage 1 with fused requantisation, stage 2, and for `reduce` the weighted top-k
  * reduce), for hosts where crossing into the library once per kernel costs more than the kernels do.  All

@@ -1,4 +1,5 @@
-"""Which cluster size shares the K range of a tile (host-only query; no GPU needed when the residency is given)."""
+"""Which cluster size shares the K range of a tile, and which launches merge row blocks (host-only queries; no GPU
+needed when the residency is given)."""
 import ctypes
 
 import pytest
@@ -42,3 +43,36 @@ def test_wait_accounting_is_not_read_for_the_cluster_kernel():
     assert "moe_gemm_split_kernel" in bench.shared_k_note(lib, one_token, 16, 2, res)
     assert bench.shared_k_note(lib, one_token, 16, 1, res) is None            # 224 tiles fill the GPU
     assert [bench.shared_k_note(lib, prefill, 128, s, res) for s in (1, 2)] == [None, None]
+
+
+TINY, MID, WIDE, MANY = (1024, 512, 8, 2), (2048, 1024, 64, 6), (4096, 14336, 8, 2), (7168, 2048, 256, 8)
+
+
+@pytest.mark.parametrize("dims,tokens,tile_m,merged", [
+    # one or two rounds of row blocks: merged, they are one round of tiles several times as long (measured 1.2-1.6x slower)
+    (TINY, 64, 16, (0, 0)), (TINY, 192, 16, (0, 0)), (TINY, 192, 32, (0, 0)), (TINY, 512, 16, (0, 0)), (TINY, 768, 64, (0, 0)),
+    # several rounds become one
+    (TINY, 1024, 16, (1, 1)), (TINY, 2048, 32, (1, 1)), (MID, 512, 16, (1, 1)), (MID, 1024, 64, (1, 1)), (WIDE, 128, 32, (1, 1)),
+    # hardly an expert has a second block, and no round is saved
+    (MID, 273, 32, (0, 0)), (MID, 546, 64, (0, 0)),
+    # weight streaming: the busy experts of skewed routing
+    (MANY, 777, 32, (1, 1)), (MANY, 1024, 64, (1, 1)),
+    # nothing to merge
+    (MANY, 4096, 128, (0, 0)),
+])
+def test_row_blocks_are_merged_where_it_saves_rounds(dims, tokens, tile_m, merged):
+    H, I, E, k = dims
+    blocks = (tokens * k + E * tile_m - k + tile_m - 1) // tile_m
+    lib = _lib.load()
+    got = (lib.flymoe_gemm_merges_blocks(1, tokens, k, E, I, H, blocks, tile_m,
+                                         _lib.ROWS_BY_TOKEN if tile_m <= 32 else _lib.ROWS_SORTED, 148),
+           lib.flymoe_gemm_merges_blocks(2, tokens, k, E, H, I, blocks, tile_m, _lib.ROWS_SORTED, 148))
+    assert got == merged
+
+
+def test_only_launches_that_the_tile_table_covers_are_merged():
+    H, I, E, k = MANY
+    lib = _lib.load()
+    assert lib.flymoe_gemm_merges_blocks(2, 8192, k, E, H, I, 4096, 16, _lib.ROWS_SORTED, 148) == 1
+    assert lib.flymoe_gemm_merges_blocks(2, 8192, k, E, H, I, 4097, 16, _lib.ROWS_SORTED, 148) == 0
+    assert lib.flymoe_gemm_merges_blocks(2, 8192, 1, 1, H, I, 512, 16, _lib.ROWS_SORTED, 148) == 0      # one expert: dense
