@@ -10,8 +10,9 @@
 //   warp 1      (leader) MMA issuer: four M=256 N=256 MMAs per K block into one of two TMEM stages.
 //   warp 2      store warp: one bulk store / bulk reduction per finished output row.
 //   warps 4-19  epilogue: four warpgroups; each thread owns one row and 2 x 32 of the tile's columns.
-// Measured on one B200, M=4096 N=K=7168 (bytes): fp8 165 us (2554 TFLOP/s) against 191 for the one-CTA kernel, bf16
-// 159 us (1320 TFLOP/s) against 187; cuBLAS 158 and 153.  Block scaling stays with the one-CTA kernel: there the
+// Measured on one B200 (bench.py --tokens 2048 --experts 8 --scaling pertoken --tile-m 128 [--in-dtype bf16]; 16384 rows,
+// 4096 x 7168 and 7168 x 2048): fp8 333 us (2887 TFLOP/s) and 212 us (2273) against 355 and 315 for the one-CTA kernel,
+// bf16 654 us (1470 TFLOP/s) and 352 us (1367) against 702 and 422.  Block scaling stays with the one-CTA kernel: there the
 // epilogue is the bound (a 16-warp variant of this kernel took 245 us against 242, and the T=4096 layer, whose 256-row
 // tiles are half empty, 4.5 ms against 3.4).
 //
@@ -435,14 +436,15 @@ static int launch_pair(const GemmArgs& a, const CUtensorMap& map_a, const CUtens
   return FLYMOE_OK;
 }
 
-// Per-token scaling, rows in sorted order, and experts that fill most of a 128-row half on average: below that the
-// second CTA of a pair would mostly idle.  At 176 rows per expert (333 tokens, 17 experts, top-9, 64-row blocks) the
-// two stages take 172 us against 227 on the one-CTA kernel, at 256 (1024 tokens, 8 experts, top-2, bf16, 128-row
-// blocks) 1044 against 1179.
+// Per-token scaling, rows in sorted order, and experts that nearly fill a 128-row half on average: below that the second
+// CTA of most pairs idles, above it the one-CTA kernel needs a second tile.  Both stages with their gathers against the
+// one-CTA kernel, even routing, experts of 4096 x 2048, 7168 x 2048, 4096 x 14336 and 2048 x 1024, fp8 and bf16, 64- and
+// 128-row blocks: 96 and 112 rows per expert 0.96-1.19 of its time (384 tokens, 8 experts of 4096 x 14336: 329 us there,
+// 390 here), 120 rows 0.90-1.04, 128 rows 0.84-1.00, 136 rows 0.80-0.89, 512 rows 0.80-0.95.
 bool use_pair_kernel(const GemmArgs& a) {
   if (a.scaling != FLYMOE_SCALE_PER_TOKEN || a.tile_m < 64 || a.a_layout != FLYMOE_ROWS_SORTED) return false;
   if (a.size_expert_ids > kTileTable) return false;
-  return (long long)a.num_tokens * a.topk >= 96LL * a.experts;
+  return (long long)a.num_tokens * a.topk >= 120LL * a.experts;
 }
 
 int launch_gemm_pair(int stage, const GemmArgs& a, int ctas, cudaStream_t stream) {

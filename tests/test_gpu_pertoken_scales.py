@@ -12,7 +12,7 @@ from tests.gpu_common import assert_close
 
 pytestmark = pytest.mark.gpu
 E, K, N = 4, 1152, 256
-# route -> tokens, row block: few tiles of long K share K in a cluster; 128-row blocks do not; 96 rows per expert and
+# route -> tokens, row block: few tiles of long K share K in a cluster; 128-row blocks do not; 120 rows per expert and
 # more run on CTA pairs
 ROUTES = {"split": (5, 16), "one-cta": (40, 128), "pair": (300, 64)}
 
