@@ -14,8 +14,8 @@
 //   warp 3      row gather (only when the activations are not in sorted-row order): copies the
 //               tile's A rows, picked through the sorted-id list, into the ring with cp.async
 //               (16 bytes per request, the 128-byte swizzle applied by hand), two K blocks in
-//               flight; the TMA producer then fetches the weights only.  Meant for row blocks
-//               of 16 or 32 rows; larger ones are gathered ahead of the launch.
+//               flight; the TMA producer then fetches the weights only.  Row blocks of 16 or
+//               32 rows (merged ones included); larger blocks are gathered ahead of the launch.
 //   warps 4-11  epilogue, two warpgroups.  Each thread owns one sorted row (its TMEM lane)
 //               and 128 of the tile's 256 accumulator columns.
 //
@@ -39,6 +39,8 @@
 // bulk-stores per-pair rows for a later top-k reduce, or (ROW_DST instantiation) stores
 // each row to a caller-given address, which may be in a peer GPU's memory.  The same
 // kernel with one expert and identity routing is the dense block-scaled GEMM.
+//
+// MERGE instantiations run an expert's consecutive row blocks of 16, 32 or 64 rows as one tile of up to 128.
 //
 // Two other kernels take what this one is not good at: gemm_split.cu launches with few tiles (a
 // cluster of CTAs shares K), gemm_pair.cu per-token scaling with many rows per expert (CTA pairs).
@@ -458,8 +460,8 @@ moe_gemm_sm100_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
       // hides behind the loop), stage 1 after the loop (measured: no spills either way, `-Xptxas -v`).
       float wgt = 1.f;
       if (STAGE == 2 && a.doweight && valid) wgt = __ldg(a.sorted_weights + r);
-      // a warp whose 32 rows are all padding has nothing to fold in (layer of 4096 tokens over 256 experts, whose second
-      // row blocks hold a dozen rows: 3381 -> 3335 us)
+      // a warp whose 32 rows are all padding has nothing to fold in (4096 tokens over 256 experts, whose second row blocks
+      // hold a dozen rows: within the spread of two runs, 0.5 %; it leaves the FMA pipe to the other warps)
       const bool work = warp_active && half_ok && __any_sync(0xffffffffu, valid);
       // stage 1: first half = gate columns, second half = up columns; stage 2: two halves of 128 columns
       const uint32_t tcol0 = tmem_base + lane_base + (STAGE == 1 ? uint32_t(wg * 64) : uint32_t(wg * 128));
