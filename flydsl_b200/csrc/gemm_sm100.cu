@@ -880,11 +880,12 @@ static double tile_rounds_us(double tiles, double rows, bool gather, int KB, int
 // Zipf, its first stage merged: 390 -> 323; 128 tokens over 256 experts of 7168 x 2048, 16-row blocks: 691 -> 315).
 static bool merge_blocks(int stage, const GemmArgs& a, int ctas) {
   if (a.tile_m >= BM || a.row_dst != nullptr || a.size_expert_ids > kTileTable || a.experts < 2) return false;
+  const int ntiles = stage == 1 ? a.n_dim / 128 : ceil_div(a.n_dim, BN);
+  if ((long long)a.size_expert_ids * ntiles <= ctas) return false;      // one round, however the rows fall
   const long long rows = (long long)a.num_tokens * a.topk;
   const long long weight_bytes = (stage == 1 ? 2LL : 1LL) * a.n_dim * a.k_dim * a.experts;
   if (weight_bytes >= (512LL << 20) && 4 * rows >= (long long)a.tile_m * a.experts) return true;
   const double mean = double(rows) / a.experts;
-  const int ntiles = stage == 1 ? a.n_dim / 128 : ceil_div(a.n_dim, BN);
   const double blocks = row_tiles(mean, a.tile_m), tiles = row_tiles(mean, BM);
   const bool gather = a.a_layout != FLYMOE_ROWS_SORTED;
   const double apart = tile_rounds_us(blocks * a.experts * ntiles, a.tile_m, gather, a.k_dim / BK, ctas);
@@ -899,7 +900,10 @@ static bool merge_blocks(int stage, const GemmArgs& a, int ctas) {
 int choose_ksplit(int stage, const GemmArgs& a) {
   // a caller that leaves other kernels some SMs gets no clusters
   if (g_cta_limit > 0 && g_cta_limit < sm_count()) return 1;
-  int clusters[kClusterSizes] = {sm_count()};
+  // no more than SMs / s clusters of s run at once: where they would not pay, the real numbers need not be asked for
+  const int sms = sm_count();
+  int clusters[kClusterSizes] = {sms, sms / 2, sms / 4, sms / 8};
+  if (plan_ksplit(stage, a, clusters) == 1) return 1;
   split_residency(stage, a.scaling, clusters);
   return plan_ksplit(stage, a, clusters);
 }

@@ -452,10 +452,8 @@ static cudaLaunchConfig_t split_config(int split, cudaLaunchAttribute* attr) {
 // Clusters of `split` CTAs that fit on the GPU at once (asked for once per device and cluster size); 0 where such a
 // cluster cannot be scheduled at all, as in a context limited to part of the GPU.
 template <int STAGE, int SCALING>
-static int resident_clusters(int split) {
+static int resident_clusters(int dev, int split) {
   static std::atomic<int> known[64][9];                    // answer + 1
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
   int n = known[dev][split].load(std::memory_order_relaxed) - 1;
   if (n >= 0) return n;
   auto* kernel = moe_gemm_split_kernel<STAGE, SCALING>;
@@ -477,7 +475,9 @@ static int launch_split(const GemmArgs& a, const CUtensorMap& map_a, const CUten
   FLYMOE_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSplitSmem)));
   const int ntiles = STAGE == 1 ? a.n_dim / 128 : ceil_div(a.n_dim, BN);
   const long long tiles = (long long)a.size_expert_ids * ntiles;
-  const int resident = resident_clusters<STAGE, SCALING>(split);     // at least one, or the plan would not say `split`
+  int dev = 0;
+  FLYMOE_CUDA_CHECK(cudaGetDevice(&dev));
+  const int resident = resident_clusters<STAGE, SCALING>(dev, split);    // at least one, or the plan would not say `split`
   cudaLaunchAttribute attr;
   cudaLaunchConfig_t cfg = split_config<STAGE, SCALING>(split, &attr);
   cfg.gridDim = dim3(unsigned((tiles < resident ? int(tiles) : resident) * split));
@@ -496,10 +496,13 @@ int launch_gemm_split(int stage, const GemmArgs& a, const CUtensorMap& map_a, co
 }
 
 void split_residency(int stage, int scaling, int* clusters) {
+  int dev = 0;
+  const bool known = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < 64;
   for (int i = 1, s = 2; i < kClusterSizes; ++i, s *= 2)
-    clusters[i] = scaling == FLYMOE_SCALE_PER_TOKEN
-                      ? (stage == 1 ? resident_clusters<1, kScalePerToken>(s) : resident_clusters<2, kScalePerToken>(s))
-                      : (stage == 1 ? resident_clusters<1, kScaleBlock128>(s) : resident_clusters<2, kScaleBlock128>(s));
+    clusters[i] = !known ? 0
+                : scaling == FLYMOE_SCALE_PER_TOKEN
+                    ? (stage == 1 ? resident_clusters<1, kScalePerToken>(dev, s) : resident_clusters<2, kScalePerToken>(dev, s))
+                    : (stage == 1 ? resident_clusters<1, kScaleBlock128>(dev, s) : resident_clusters<2, kScaleBlock128>(dev, s));
 }
 
 int plan_ksplit(int stage, const GemmArgs& a, const int* clusters) {

@@ -232,19 +232,22 @@ class FusedMoEBlockscale:
         _lib.check(self.lib.flymoe_moe_layer(args, stream), "moe_layer")
         return out[:T] if out.shape[0] != T else out
 
-    def _pieces_unchanged(self) -> bool:
-        """No subclass or caller has put its own gate or experts_forward, or another way to fetch rows, in place."""
-        cls, own = type(self), self.__dict__
-        return (cls.gate is FusedMoEBlockscale.gate and cls.experts_forward is FusedMoEBlockscale.experts_forward
-                and "gate" not in own and "experts_forward" not in own
-                and self.gather_in_kernel == (self.tile_m <= 32))
+    # forward() may take the one-call path: no subclass has a gate or experts_forward of its own
+    _own_pieces = True
+
+    def __init_subclass__(cls, **kwargs):
+        super().__init_subclass__(**kwargs)
+        cls._own_pieces = (cls.gate is FusedMoEBlockscale.gate
+                           and cls.experts_forward is FusedMoEBlockscale.experts_forward)
 
     def forward(self, logits: torch.Tensor, xq: torch.Tensor, x_scale_t: torch.Tensor,
                 out: torch.Tensor | None = None, stream=None) -> torch.Tensor:
         """logits [T, E] (f32/f16/bf16), xq e4m3 [T, H], x_scale_t f32 [H/128, T] -> out [T, H]."""
         tokens = logits.shape[0]
         h = _lib.stream_handle(stream)
-        if self.stage2_mode != "rows" and self.timing_events is None and self._pieces_unchanged():
+        own = self.__dict__                        # a piece, or the way to fetch rows, may be replaced on the object too
+        if (self.stage2_mode != "rows" and self.timing_events is None and self._own_pieces and "gate" not in own
+                and "experts_forward" not in own and self.gather_in_kernel == (self.tile_m <= 32)):
             return self._forward_once(logits, xq, x_scale_t, tokens, out, h)
         self.gate(logits, tokens, h)
         res = self.experts_forward(self.topk_ids, self.topk_weights, xq, x_scale_t, tokens, h, out)
